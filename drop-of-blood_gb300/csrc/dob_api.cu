@@ -542,11 +542,19 @@ dob_status dob_create(const dob_config* cfg, dob_ctx** out) {
     L.d = make_grid(s.g.nx >> l, s.g.ny >> l, s.g.nz >> l);
     const float sc = (float)s.g.nx / (float)L.d.nx;
     L.h2 = sc * sc;
-    if (l == 0) { L.e = s.p; L.b = s.rhs; continue; }
+    const bool leg = l < s.nlev - 1 && mg_leg_level(L.d);
+    if (l == 0) {
+      L.e = s.p;
+      L.b = s.rhs;
+      if (leg && s.prec != DOB_PREC_MIXED) A((void**)&L.e2, L.d.n() * 4);
+      continue;
+    }
     if (s.prec == DOB_PREC_MIXED && l >= kMixedBF16Level) {
       A((void**)&L.eh, L.d.n() * 2); A((void**)&L.bh, L.d.n() * 2);
+      if (leg) A((void**)&L.eh2, L.d.n() * 2);
     } else {
       A((void**)&L.e, L.d.n() * 4); A((void**)&L.b, L.d.n() * 4);
+      if (leg) A((void**)&L.e2, L.d.n() * 4);
     }
   }
   if (s.prec == DOB_PREC_MIXED) {

@@ -24,6 +24,10 @@ struct MgLevel {
   float* b;            // right-hand side (levels >= 1), FP32
   __nv_bfloat16* eh;   // BF16 arrays used by the mixed-precision inner solve
   __nv_bfloat16* bh;
+  // second array of a level whose legs run in one launch each (mg_leg_level):
+  // level 0: the smoothed pressure between the legs, else the level's result
+  float* e2;
+  __nv_bfloat16* eh2;
 };
 
 // Red-black split index of cell (x,y,z): colour c = (x+y+z)&1 selects the
@@ -341,8 +345,12 @@ constexpr int kDenseCoarseTarget = 2304;
 std::vector<float> coarse_inverse(const Grid& c, float h2, int ref);
 
 // ---- launchers (k_mg.cu) ---------------------------------------------------------------
-// Raise the dynamic shared-memory limit of the coarse-grid kernel (once per process).
+// Raise the dynamic shared-memory limits of the coarse-grid and leg kernels
+// (once per device).
 cudaError_t mg_prepare();
+// Whether a level of this size runs each leg of the V-cycle in one launch
+// (it then needs its second array, MgLevel::e2 / eh2).
+bool mg_leg_level(const Grid& d);
 void launch_pressure_solve(const DevState& s, cudaStream_t st);
 void launch_residual_norm(const DevState& s, double* out, cudaStream_t st);
 // mean removal: launch_sum leaves per-block partials in part (kSumBlocks

@@ -57,9 +57,11 @@ constexpr size_t kAlign = 256;
 constexpr size_t kSlotBytes = 1024;  // FP64 + u32 reduction slots at the front
 constexpr size_t kPartBytes = PART_SLOTS * kSumBlocks * sizeof(double);  // mean-removal partials
 // Layout for n cells: slots, partials, split p (4n), split rhs (4n), then correction and
-// right-hand side of every coarser grid, each rounded up to 256 bytes.  The
-// coarser grids hold fewer than n/7 cells together, so 10 bytes per cell
-// bounds the whole layout for every accepted grid.
+// right-hand side of every coarser grid and the second array of each small
+// level (mg_leg_level), each rounded up to 256 bytes.  The coarser grids hold
+// fewer than n/7 cells together, 12 bytes each at most, so 10 bytes per cell
+// of the largest accepted grid bound the whole layout for every accepted grid
+// (the finest grid itself has a second array only when small).
 // The dense inverse of an exactly solved coarsest grid (up to
 // kNoAllocDenseMax cells, the closed-box configuration's target) follows the
 // multigrid arrays.
@@ -191,13 +193,16 @@ extern "C" dob_status dob_pressure_solve_noalloc(const dob_config* cfg, const fl
     L.d = make_grid(s.g.nx >> l, s.g.ny >> l, s.g.nz >> l);
     const float sc = (float)s.g.nx / (float)L.d.nx;
     L.h2 = sc * sc;
+    const bool leg = l < s.nlev - 1 && mg_leg_level(L.d);
     if (l == 0) {
       L.e = s.p;
       L.b = s.rhs;
+      if (leg) L.e2 = take(n);
       continue;
     }
     L.e = take(L.d.n());
     L.b = take(L.d.n());
+    if (leg) L.e2 = take(L.d.n());
   }
   if (cfg->mg_coarse_sweeps < 0) {
     // The coarsest grid's inverse sits at the end of the array.  It is

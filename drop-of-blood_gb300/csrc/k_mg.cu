@@ -22,13 +22,14 @@
 //                       never stored)
 //   k_prolong_add2      e_f += trilinear(e_c), cell-centred, two coarse cells
 //                       per thread
-//   k_coarse_dense      exact coarsest solve e = M b with a precomputed dense
-//                       (pseudo-)inverse
-//   k_coarse_cluster    every sweep of the coarsest grid inside one
-//                       thread-block cluster: each CTA keeps a slab of planes in
-//                       shared memory, reads the neighbour slabs' boundary
-//                       planes through distributed shared memory, and the
-//                       half-sweeps are separated by hardware cluster barriers
+//   k_leg_down, k_leg_up  the whole way down or up of a small level in one
+//                       launch (dob_mgleg.cuh)
+//   k_coarse_dense_pre  exact coarsest solve e = M b with a precomputed dense
+//   (k_coarse_dense)    (pseudo-)inverse
+//   k_coarse_sweeps     every sweep of the coarsest grid in one launch: one CTA,
+//                       or a cluster whose CTAs hold a slab each and store
+//                       their boundary planes into their neighbours' shared
+//                       memory, one hardware barrier per half-sweep
 //   k_defect_df4        residual of the pressure (double-float in the mixed
 //   (k_defect_df)       mode) formed with error-free FP32 transformations, its
 //                       max and norm (statistics and the mixed defect loop)
@@ -54,6 +55,10 @@ template <> __device__ __forceinline__ float as_stored<__nv_bfloat16>(float v) {
 }
 
 __device__ __forceinline__ bool skip_now(const unsigned int* skip) { return skip != nullptr && *skip != 0u; }
+
+}  // namespace dob
+#include "dob_mgleg.cuh"
+namespace dob {
 
 // evalMgStencil (fluid.ts:568-602) on a red-black split array: neighbour sum
 // and diagonal count in the order x-, x+, y-, y+, z-, z+.  Reference BCs
@@ -572,6 +577,51 @@ __global__ void __launch_bounds__(1024) k_coarse_dense(Grid d, const float* __re
   }
 }
 
+// The same solve for n <= 32 kDenseChain cells: a CTA of 256 threads forms 8
+// rows, thread (w, r) the sum over i = w, w + 32, ... of row r, in the same
+// order.  M does not change, so each thread loads its up to kDenseChain
+// elements of it (the whole matrix, spread over the registers of n/8 CTAs)
+// before waiting for the restriction that forms b; after it only b, 2304
+// shared-memory multiply-adds and the 32 partial sums are left.
+// 12x16x12 cells: the solve costs a step of 48x64x48 (four cycles) 182 -> 179 us.
+constexpr int kDenseChain = 72;
+template <class T>
+__global__ void __launch_bounds__(256, 2) k_coarse_dense_pre(Grid d, const float* __restrict__ M, int n,
+                                                             T* __restrict__ e, const T* __restrict__ b,
+                                                             const unsigned int* __restrict__ skip) {
+  __shared__ float sbv[32 * kDenseChain];
+  __shared__ float part[32 * 8];
+  const int r = threadIdx.x & 7, w = threadIdx.x >> 3;
+  const int j = blockIdx.x * 8 + r;
+  float m[kDenseChain];
+#pragma unroll
+  for (int k = 0; k < kDenseChain; ++k) {
+    const int i = w + 32 * k;
+    m[k] = i < n && j < n ? __ldg(M + (uint32_t)i * (uint32_t)n + (uint32_t)j) : 0.0f;
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (skip_now(skip)) return;
+  for (int i = threadIdx.x; i < n; i += 256) {
+    const int x = i % d.nx, row = i / d.nx, y = row % d.ny, z = row / d.ny;
+    sbv[i] = ldv(b + rb_index(d, x, y, z));
+  }
+  __syncthreads();
+  float acc = 0.0f;
+#pragma unroll
+  for (int k = 0; k < kDenseChain; ++k)
+    if (w + 32 * k < n) acc = fmaf(m[k], sbv[w + 32 * k], acc);
+  part[w * 8 + r] = acc;
+  __syncthreads();
+  if (threadIdx.x < 8 && j < n) {
+    float sum = part[r];
+#pragma unroll
+    for (int k = 1; k < 32; ++k) sum += part[k * 8 + r];
+    const int x = j % d.nx, row = j / d.nx, y = row % d.ny, z = row / d.ny;
+    stf(e + rb_index(d, x, y, z), sum);
+  }
+}
+
 template <class T>
 __global__ void k_fill_zero(T* __restrict__ a, size_t n, const unsigned int* __restrict__ skip) {
   pdl_wait();
@@ -581,68 +631,114 @@ __global__ void k_fill_zero(T* __restrict__ a, size_t n, const unsigned int* __r
     a[i] = T(0.0f);
 }
 
-// MG_COARSE_SOLVE_L3 (fluid.ts:687-739) spread over a thread-block cluster of
-// CS CTAs: CTA r owns z-planes [r*pz, (r+1)*pz) of the coarsest grid (pz =
-// nz/CS) in its shared memory (natural layout), zero start, `sweeps` sweeps.
-// Neighbouring planes of other CTAs are read through distributed shared
-// memory; every half-sweep ends with a cluster barrier, so a colour only
-// ever reads the other colour's finished values, exactly like the
-// reference's single-workgroup solve.
+// MG_COARSE_SOLVE_L3 (fluid.ts:687-739): every sweep of the coarsest grid,
+// from zero, in one launch of CS CTAs (one, or a thread-block cluster): CTA r
+// owns planes [r nz / CS, (r + 1) nz / CS) in its shared memory, red-black
+// split like the arrays, with one word, row and plane of padding around them.
+// The padding holds the zeros of the grid's outside, and between CTAs copies
+// of the neighbours' boundary planes: whoever updates a boundary plane stores
+// it into the neighbour's padding too (distributed shared memory), so every
+// read is local and the half-sweeps need one barrier each; a colour only ever
+// reads the other colour's finished values, exactly like the reference's
+// single-workgroup solve.
+// A thread's at most kCoarseCells cells of either colour keep their addresses,
+// diagonals and right-hand sides in registers: 6552 cells, 6 sweeps, in 15 us
+// where two CTAs that formed them from the index on every update took 31.
+constexpr int kCoarseThreads = 1024, kCoarseCells = 4;
+constexpr size_t kCoarseSmem = 220 * 1024;  // dynamic shared memory, at most
+__host__ __device__ inline size_t coarse_words(const Grid& d, int cs) {  // shared floats per CTA
+  const size_t pz = (d.nz + cs - 1) / cs, hx = d.nx / 2;
+  return 2 * (hx + 2) * (d.ny + 2) * (pz + 2);
+}
+inline bool coarse_fits(const Grid& d, int cs) {
+  const size_t pz = (d.nz + cs - 1) / cs;
+  return d.nz >= cs && (size_t)(d.nx / 2) * d.ny * pz <= (size_t)kCoarseThreads * kCoarseCells &&
+         coarse_words(d, cs) * sizeof(float) <= kCoarseSmem;
+}
 template <class T, int CS>
-__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(512)
-    k_coarse_cluster(Grid d, float h2, int ref, int sweeps, T* __restrict__ e, const T* __restrict__ b,
-                     const unsigned int* __restrict__ skip) {
+__global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(kCoarseThreads)
+    k_coarse_sweeps(Grid d, float h2, int ref, int sweeps, T* __restrict__ e, const T* __restrict__ b,
+                    const unsigned int* __restrict__ skip) {
+  cg::cluster_group cl = cg::this_cluster();
+  extern __shared__ float csm[];  // [2][pzm + 2][ny + 2][hx + 2]
+  const int rank = (int)blockIdx.x % CS;
+  const int z0 = rank * d.nz / CS, pz = (rank + 1) * d.nz / CS - z0;
+  const int hx = d.nx >> 1, kw = hx + 2, pl = kw * (d.ny + 2);
+  const int ehalf = ((d.nz + CS - 1) / CS + 2) * pl;
+  const int ncol = pz * d.ny * hx;  // cells of one colour here
+  for (int i = threadIdx.x; i < 2 * ehalf; i += kCoarseThreads) csm[i] = 0.0f;
+  // cell q: address in a padded half, x parity of its red cell, and the
+  // diagonals of its cells of x parity 0 and 1
+  int at[kCoarseCells], par[kCoarseCells];
+  float dg[kCoarseCells][2], bv[kCoarseCells][2];
+#pragma unroll
+  for (int m = 0; m < kCoarseCells; ++m) {
+    const int q = (int)threadIdx.x + m * kCoarseThreads;
+    const int k = q % hx, row = q / hx, y = row % d.ny, zl = row / d.ny, z = z0 + zl;
+    at[m] = (zl + 1) * pl + (y + 1) * kw + k + 1;
+    par[m] = (y + z) & 1;
+    const float dyz = 6.0f - (y == 0 ? 1.0f : 0.0f) - (y == d.ny - 1 && !ref ? 1.0f : 0.0f) - (z == 0 ? 1.0f : 0.0f) -
+                      (z == d.nz - 1 ? 1.0f : 0.0f);  // the +y face always counted with the Dirichlet top
+    dg[m][0] = dyz - (k == 0 ? 1.0f : 0.0f);
+    dg[m][1] = dyz - (k == hx - 1 ? 1.0f : 0.0f);
+  }
+  // the neighbours' padding planes that mirror this CTA's boundary planes,
+  // as offsets from a cell of the boundary plane
+  float *dn = nullptr, *up = nullptr;
+  if (CS > 1) {
+    if (rank > 0) {
+      const int pzd = z0 - (rank - 1) * d.nz / CS;
+      dn = cl.map_shared_rank(csm, rank - 1) + pzd * pl;
+    }
+    if (rank < CS - 1) up = cl.map_shared_rank(csm, rank + 1) - pz * pl;
+  }
   pdl_wait();
   pdl_trigger();
-  cg::cluster_group cl = cg::this_cluster();
-  extern __shared__ float csm[];
-  const int rank = (int)cl.block_rank();
-  const int pz = d.nz / CS;
-  const int plane = d.nx * d.ny;
-  const int nloc = pz * plane;
-  float* se = csm;
-  float* sb = csm + nloc;
   const bool skipping = skip_now(skip);  // uniform: every CTA takes the same path
-  const int z0 = rank * pz;
-  for (int k = threadIdx.x; k < nloc; k += blockDim.x) {
-    const int zl = k / plane, rem = k - zl * plane;
-    const int y = rem / d.nx, x = rem - y * d.nx;
-    se[k] = 0.0f;
-    sb[k] = skipping ? 0.0f : rb_at(b, d, x, y, z0 + zl);
+  const uint32_t half = (uint32_t)(d.n() >> 1), base = (uint32_t)z0 * d.ny * hx;
+#pragma unroll
+  for (int m = 0; m < kCoarseCells; ++m) {
+    const int q = (int)threadIdx.x + m * kCoarseThreads;
+    const bool on = q < ncol && !skipping;
+    bv[m][0] = on ? ldv(b + base + q) : 0.0f;
+    bv[m][1] = on ? ldv(b + half + base + q) : 0.0f;
   }
-  const float* below = rank > 0 ? cl.map_shared_rank(se, rank - 1) + (pz - 1) * plane : nullptr;
-  const float* above = rank < CS - 1 ? cl.map_shared_rank(se, rank + 1) : nullptr;
-  cl.sync();
+  if (CS > 1) cl.sync();  // every CTA has cleared its padding
+  else __syncthreads();
   const int nsw = skipping ? 0 : sweeps;
   for (int s = 0; s < nsw; ++s) {
+#pragma unroll
     for (int color = 0; color < 2; ++color) {
-      const int hxc = d.nx >> 1;
-      for (int q = threadIdx.x; q < (nloc >> 1); q += blockDim.x) {  // the cells of this colour
-        const int row = q / hxc, kx = q - row * hxc;
-        const int zl = row / d.ny, y = row - zl * d.ny;
-        const int z = z0 + zl;
-        const int x = 2 * kx + ((y + z + color) & 1);
-        const int rem = y * d.nx + x;
-        const int k = zl * plane + rem;
-        float sumN = 0.0f, diag = ref ? 1.0f : 0.0f;
-        if (x > 0) { sumN = sumN + se[k - 1]; diag = diag + 1.0f; }
-        if (x < d.nx - 1) { sumN = sumN + se[k + 1]; diag = diag + 1.0f; }
-        if (y > 0) { sumN = sumN + se[k - d.nx]; diag = diag + 1.0f; }
-        if (y < d.ny - 1) { sumN = sumN + se[k + d.nx]; if (!ref) diag = diag + 1.0f; }
-        if (z > 0) { sumN = sumN + (zl > 0 ? se[k - plane] : below[rem]); diag = diag + 1.0f; }
-        if (z < d.nz - 1) { sumN = sumN + (zl < pz - 1 ? se[k + plane] : above[rem]); diag = diag + 1.0f; }
-        se[k] = as_stored<T>((sumN - h2 * sb[k]) / diag);
+      float* own = csm + color * ehalf;
+      const float* oth = csm + (1 - color) * ehalf;
+#pragma unroll
+      for (int m = 0; m < kCoarseCells; ++m) {
+        const int q = (int)threadIdx.x + m * kCoarseThreads;
+        if (q < ncol) {
+          const int p = par[m] ^ color;
+          const float* o = oth + at[m];
+          const float sumN = ((((o[p - 1] + o[p]) + o[-kw]) + o[kw]) + o[-pl]) + o[pl];
+          const float v = as_stored<T>((sumN - h2 * bv[m][color]) / (p ? dg[m][1] : dg[m][0]));
+          own[at[m]] = v;
+          if (CS > 1) {
+            if (at[m] < 2 * pl && dn) dn[color * ehalf + at[m]] = v;
+            if (at[m] >= pz * pl && up) up[color * ehalf + at[m]] = v;
+          }
+        }
       }
-      cl.sync();
+      if (CS > 1) cl.sync();
+      else __syncthreads();
     }
   }
-  if (!skipping)
-    for (int k = threadIdx.x; k < nloc; k += blockDim.x) {
-      const int zl = k / plane, rem = k - zl * plane;
-      const int y = rem / d.nx, x = rem - y * d.nx;
-      stf(e + rb_index(d, x, y, z0 + zl), se[k]);
+  if (skipping) return;  // after the cluster's only barrier
+#pragma unroll
+  for (int m = 0; m < kCoarseCells; ++m) {
+    const int q = (int)threadIdx.x + m * kCoarseThreads;
+    if (q < ncol) {
+      stf(e + base + q, csm[at[m]]);
+      stf(e + half + base + q, csm[ehalf + at[m]]);
     }
-  cl.sync();  // keep this CTA's shared memory alive until its neighbours are done reading it
+  }
 }
 
 // ---- FP64 pieces ---------------------------------------------------------------------
@@ -1128,19 +1224,84 @@ void launch_split(const float* src, float* dst, const Grid& d, bool to_split, cu
   else k_from_split<<<g_cells(d), b_cells(), 0, st>>>(src, dst, d);
 }
 
+// ---- one launch per leg (dob_mgleg.cuh) ----
+// Levels of up to half a million cells: there a leg's redundant halo work
+// costs less than the launches it saves (level of 72x104x56 = 419k cells:
+// 254 against 263 us a step); at 1.2 million (96x128x96) the launch chain,
+// which does no work twice, is faster (257 against 302 us a step).
+constexpr size_t kLegMaxCells = 500000;
+bool mg_leg_level(const Grid& d) { return d.n() <= kLegMaxCells; }
+template <class L> static dim3 leg_grid(const Grid& d) {
+  return dim3((d.nx + L::TX - 1) / L::TX, (d.ny + L::TY - 1) / L::TY, (d.nz + L::TZ - 1) / L::TZ);
+}
+// Regions 16 cells wide where every block then has an SM to itself (a block
+// of half the threads finishes sooner: 24x32x24 and smaller), else 32, whose
+// halo is the smaller part of it (48x64x48: 129 against 149 us of solve a step).
+template <int S> static bool leg_narrow(const DevState& s, const Grid& d) {
+  const dim3 g = leg_grid<LegTile<8, S>>(d);
+  return (int)(g.x * g.y * g.z) <= s.num_sms;
+}
+template <class T, class TC, class L>
+static void leg_down_l(const DevState& s, int l, const T* a, const T* b, T* out, TC* bc, const unsigned int* skip,
+                       cudaStream_t st) {
+  const MgLevel& V = s.lv[l];
+  auto run = [&](auto* k) {
+    launch_pdl(k, leg_grid<L>(V.d), dim3(L::NT), 0, st, V.d, s.lv[l + 1].d, V.h2, 1.0f / V.h2, s.ref, a, b, out, bc,
+               skip);
+  };
+  if (!a) run(k_leg_down<T, TC, L, true>);
+  else if constexpr (sizeof(T) == 4 && sizeof(TC) == 4) run(k_leg_down<T, TC, L, false>);
+}
+template <class T, class TC, class L>
+static void leg_up_l(const DevState& s, int l, const T* a, const T* b, const TC* ec, T* out, const unsigned int* skip,
+                     cudaStream_t st) {
+  const MgLevel& V = s.lv[l];
+  launch_pdl(k_leg_up<T, TC, L>, leg_grid<L>(V.d), dim3(L::NT), 0, st, V.d, s.lv[l + 1].d, V.h2, s.ref, a, b, ec, out,
+             skip);
+}
+// Level l's pre-smoothing (from zero: a null; else FP32 with its first red
+// half-sweep just done, in a) and restriction, and its prolongation and
+// post-smoothing; 1 or 2 sweeps.
+template <class T, class TC>
+static void leg_down(const DevState& s, int l, const T* a, const T* b, T* out, TC* bc, int sweeps,
+                     const unsigned int* skip, cudaStream_t st) {
+  const Grid& d = s.lv[l].d;
+  if (sweeps == 1) {
+    if (leg_narrow<1>(s, d)) leg_down_l<T, TC, LegTile<8, 1>>(s, l, a, b, out, bc, skip, st);
+    else leg_down_l<T, TC, LegTile<16, 1>>(s, l, a, b, out, bc, skip, st);
+  } else {
+    if (leg_narrow<2>(s, d)) leg_down_l<T, TC, LegTile<8, 2>>(s, l, a, b, out, bc, skip, st);
+    else leg_down_l<T, TC, LegTile<16, 2>>(s, l, a, b, out, bc, skip, st);
+  }
+}
+template <class T, class TC>
+static void leg_up(const DevState& s, int l, const T* a, const T* b, const TC* ec, T* out, int sweeps,
+                   const unsigned int* skip, cudaStream_t st) {
+  const Grid& d = s.lv[l].d;
+  if (sweeps == 1) {
+    if (leg_narrow<1>(s, d)) leg_up_l<T, TC, LegTile<8, 1>>(s, l, a, b, ec, out, skip, st);
+    else leg_up_l<T, TC, LegTile<16, 1>>(s, l, a, b, ec, out, skip, st);
+  } else {
+    if (leg_narrow<2>(s, d)) leg_up_l<T, TC, LegTile<8, 2>>(s, l, a, b, ec, out, skip, st);
+    else leg_up_l<T, TC, LegTile<16, 2>>(s, l, a, b, ec, out, skip, st);
+  }
+}
+static bool leg_sweeps_ok(int pre, int post) { return (pre == 1 || pre == 2) && (post == 1 || post == 2); }
+// the level has its second array and sweep counts that the leg kernels cover
+static bool leg_ok(const DevState& s, int l) {
+  return l < s.nlev - 1 && (s.lv[l].e2 || s.lv[l].eh2) &&
+         (l == 0 ? leg_sweeps_ok(s.pre0, s.post0) : leg_sweeps_ok(s.pre, s.post));
+}
+
 template <class T, int CS>
 static cudaError_t cluster_attr() {
-  return cudaFuncSetAttribute(k_coarse_cluster<T, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024);
+  return cudaFuncSetAttribute(k_coarse_sweeps<T, CS>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kCoarseSmem);
 }
 
 cudaError_t mg_prepare() {
   cudaError_t e = cluster_attr<float, 8>();
-  if (e == cudaSuccess) e = cluster_attr<float, 4>();
-  if (e == cudaSuccess) e = cluster_attr<float, 2>();
   if (e == cudaSuccess) e = cluster_attr<float, 1>();
   if (e == cudaSuccess) e = cluster_attr<__nv_bfloat16, 8>();
-  if (e == cudaSuccess) e = cluster_attr<__nv_bfloat16, 4>();
-  if (e == cudaSuccess) e = cluster_attr<__nv_bfloat16, 2>();
   if (e == cudaSuccess) e = cluster_attr<__nv_bfloat16, 1>();
   return e;
 }
@@ -1231,31 +1392,25 @@ static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, bool 
     }
 }
 
-template <class T, int CS>
-static void launch_cluster(const MgLevel& L, int ref, int sweeps, T* e, const T* b, const unsigned int* skip,
-                           cudaStream_t st) {
-  const size_t smem = 2 * (L.d.n() / CS) * sizeof(float);
-  launch_pdl(k_coarse_cluster<T, CS>, dim3(CS), dim3(512), smem, st, L.d, L.h2, ref, sweeps, e, b, skip);
-}
-
 template <class T>
 static void coarse_solve(const DevState& s, int l, T* e, const T* b, const unsigned int* skip, cudaStream_t st) {
   const MgLevel& L = s.lv[l];
   if (s.coarse_sweeps < 0) {  // exact: e = M b with the precomputed inverse
-    launch_pdl(k_coarse_dense<T>, dim3((s.cn + 31) / 32), dim3(1024), (s.cn + 1024) * sizeof(float), st, L.d,
-               s.cinv, s.cn, e, b, skip);
+    if (s.cn <= 32 * kDenseChain)
+      launch_pdl(k_coarse_dense_pre<T>, dim3((s.cn + 7) / 8), dim3(256), 0, st, L.d, s.cinv, s.cn, e, b, skip);
+    else
+      launch_pdl(k_coarse_dense<T>, dim3((s.cn + 31) / 32), dim3(1024), (s.cn + 1024) * sizeof(float), st, L.d,
+                 s.cinv, s.cn, e, b, skip);
     return;
   }
-  int cs = 0;
-  for (int c : {8, 4, 2, 1})
-    if (L.d.nz % c == 0 && 2 * (L.d.n() / c) * sizeof(float) <= 200 * 1024) { cs = c; break; }
-  switch (cs) {
-    case 8: launch_cluster<T, 8>(L, s.ref, s.coarse_sweeps, e, b, skip, st); break;
-    case 4: launch_cluster<T, 4>(L, s.ref, s.coarse_sweeps, e, b, skip, st); break;
-    case 2: launch_cluster<T, 2>(L, s.ref, s.coarse_sweeps, e, b, skip, st); break;
-    case 1: launch_cluster<T, 1>(L, s.ref, s.coarse_sweeps, e, b, skip, st); break;
-    default: smooth<T, T>(s, l, e, b, s.coarse_sweeps, true, nullptr, skip, st); break;
-  }
+  // one CTA where its threads hold the grid, else a cluster of eight
+  auto run = [&](auto* k, int cs) {
+    launch_pdl(k, dim3(cs), dim3(kCoarseThreads), coarse_words(L.d, cs) * sizeof(float), st, L.d, L.h2, s.ref,
+               s.coarse_sweeps, e, b, skip);
+  };
+  if (coarse_fits(L.d, 1)) run(k_coarse_sweeps<T, 1>, 1);
+  else if (coarse_fits(L.d, 8)) run(k_coarse_sweeps<T, 8>, 8);
+  else smooth<T, T>(s, l, e, b, s.coarse_sweeps, true, nullptr, skip, st);
 }
 
 // One V-cycle on (x0, b0); per-level arrays E[l], B[l] for l >= 1.
@@ -1268,20 +1423,41 @@ static void vcycle(const DevState& s, T* x0, const T* b0, T* const* E, T* const*
     smooth<T, T>(s, 0, x0, b0, s.pre + s.post, zero0, nullptr, skip, st);
     return;
   }
-  smooth<T, T>(s, 0, x0, b0, s.pre0, zero0, nullptr, skip, st);
   // each level in between starts its smoothing from zero: its first red
-  // half-sweep reads only its right-hand side, so the restriction forming
-  // that right-hand side also forms it (one launch fewer per level)
-  const bool fuse = s.pre > 0;
-  restrict_level<T>(s, 0, x0, b0, B[1], skip, st, nullptr, nullptr, fuse && L > 2 ? E[1] : nullptr);
+  // half-sweep reads only its right-hand side, so a restriction kernel forming
+  // that right-hand side also forms it (one launch fewer per level); a leg
+  // forms it itself
+  auto ered = [&](int l) { return s.pre > 0 && l < L - 1 && !leg_ok(s, l) ? E[l] : nullptr; };
+  bool red_done = false;  // the restriction into the next level formed its red half-sweep
+  const bool leg0 = leg_ok(s, 0) && !zero0;
+  if (leg0) {
+    half_sweep<T>(s, 0, 0, false, x0, b0, skip, st);
+    leg_down<T, T>(s, 0, x0, b0, s.lv[0].e2, B[1], s.pre0, skip, st);
+  } else {
+    smooth<T, T>(s, 0, x0, b0, s.pre0, zero0, nullptr, skip, st);
+    restrict_level<T>(s, 0, x0, b0, B[1], skip, st, nullptr, nullptr, ered(1));
+    red_done = ered(1) != nullptr;
+  }
+  T* X[kMaxLevels];  // each level's correction
+  for (int l = 1; l < L; ++l) X[l] = E[l];
   for (int l = 1; l < L - 1; ++l) {
-    smooth<T, T>(s, l, E[l], B[l], s.pre, true, nullptr, skip, st, fuse);
-    restrict_level<T>(s, l, E[l], B[l], B[l + 1], skip, st, nullptr, nullptr,
-                      fuse && l + 1 < L - 1 ? E[l + 1] : nullptr);
+    if (leg_ok(s, l)) {
+      leg_down<T, T>(s, l, nullptr, B[l], E[l], B[l + 1], s.pre, skip, st);
+      X[l] = s.lv[l].e2;
+      red_done = false;
+    } else {
+      smooth<T, T>(s, l, E[l], B[l], s.pre, true, nullptr, skip, st, red_done);
+      restrict_level<T>(s, l, E[l], B[l], B[l + 1], skip, st, nullptr, nullptr, ered(l + 1));
+      red_done = ered(l + 1) != nullptr;
+    }
   }
   coarse_solve<T>(s, L - 1, E[L - 1], B[L - 1], skip, st);
-  for (int l = L - 2; l >= 1; --l) smooth<T, T>(s, l, E[l], B[l], s.post, false, E[l + 1], skip, st);
-  smooth<T, T>(s, 0, x0, b0, s.post0, false, E[1], skip, st);
+  for (int l = L - 2; l >= 1; --l) {
+    if (leg_ok(s, l)) leg_up<T, T>(s, l, E[l], B[l], X[l + 1], X[l], s.post, skip, st);
+    else smooth<T, T>(s, l, E[l], B[l], s.post, false, X[l + 1], skip, st);
+  }
+  if (leg0) leg_up<T, T>(s, 0, s.lv[0].e2, b0, X[1], x0, s.post0, skip, st);
+  else smooth<T, T>(s, 0, x0, b0, s.post0, false, X[1], skip, st);
 }
 
 // ---- the mixed-precision correction solve --------------------------------------------------
@@ -1291,23 +1467,49 @@ struct MixLv {
   float *ef, *bf;
   __nv_bfloat16 *eh, *bh;
   bool h;
+  float* xf;  // the level's correction after its post-smoothing
+  __nv_bfloat16* xh;
 };
 static void mix_smooth(const DevState& s, int l, const MixLv* M, int sweeps, bool zero, bool add_coarse,
                        const unsigned int* skip, cudaStream_t st) {
   const bool ch = add_coarse && M[l + 1].h;
   if (M[l].h) {
-    smooth<__nv_bfloat16, __nv_bfloat16>(s, l, M[l].eh, M[l].bh, sweeps, zero, add_coarse ? M[l + 1].eh : nullptr,
+    smooth<__nv_bfloat16, __nv_bfloat16>(s, l, M[l].eh, M[l].bh, sweeps, zero, add_coarse ? M[l + 1].xh : nullptr,
                                          skip, st);
   } else if (ch) {
-    smooth<float, __nv_bfloat16>(s, l, M[l].ef, M[l].bf, sweeps, zero, M[l + 1].eh, skip, st);
+    smooth<float, __nv_bfloat16>(s, l, M[l].ef, M[l].bf, sweeps, zero, M[l + 1].xh, skip, st);
   } else {
-    smooth<float, float>(s, l, M[l].ef, M[l].bf, sweeps, zero, add_coarse ? M[l + 1].ef : nullptr, skip, st);
+    smooth<float, float>(s, l, M[l].ef, M[l].bf, sweeps, zero, add_coarse ? M[l + 1].xf : nullptr, skip, st);
   }
 }
 static void mix_restrict(const DevState& s, int l, const MixLv* M, const unsigned int* skip, cudaStream_t st) {
   if (M[l].h) restrict_level<__nv_bfloat16, __nv_bfloat16>(s, l, M[l].eh, M[l].bh, M[l + 1].bh, skip, st);
   else if (M[l + 1].h) restrict_level<float, __nv_bfloat16>(s, l, M[l].ef, M[l].bf, M[l + 1].bh, skip, st);
   else restrict_level<float, float>(s, l, M[l].ef, M[l].bf, M[l + 1].bf, skip, st);
+}
+// a level between the finest and the coarsest, down (smoothing from zero,
+// restriction) and up (prolongation, smoothing)
+static void mix_down(const DevState& s, int l, const MixLv* M, const unsigned int* skip, cudaStream_t st) {
+  if (!leg_ok(s, l)) {
+    mix_smooth(s, l, M, s.pre, true, false, skip, st);
+    mix_restrict(s, l, M, skip, st);
+  } else if (M[l].h) {
+    leg_down<__nv_bfloat16, __nv_bfloat16>(s, l, nullptr, M[l].bh, M[l].eh, M[l + 1].bh, s.pre, skip, st);
+  } else if (M[l + 1].h) {
+    leg_down<float, __nv_bfloat16>(s, l, nullptr, M[l].bf, M[l].ef, M[l + 1].bh, s.pre, skip, st);
+  } else {
+    leg_down<float, float>(s, l, nullptr, M[l].bf, M[l].ef, M[l + 1].bf, s.pre, skip, st);
+  }
+}
+static void mix_up(const DevState& s, int l, const MixLv* M, const unsigned int* skip, cudaStream_t st) {
+  if (!leg_ok(s, l))
+    mix_smooth(s, l, M, s.post, false, true, skip, st);
+  else if (M[l].h)
+    leg_up<__nv_bfloat16, __nv_bfloat16>(s, l, M[l].eh, M[l].bh, M[l + 1].xh, M[l].xh, s.post, skip, st);
+  else if (M[l + 1].h)
+    leg_up<float, __nv_bfloat16>(s, l, M[l].ef, M[l].bf, M[l + 1].xh, M[l].xf, s.post, skip, st);
+  else
+    leg_up<float, float>(s, l, M[l].ef, M[l].bf, M[l + 1].xf, M[l].xf, s.post, skip, st);
 }
 double smoother_pass(const DevState& s, cudaStream_t st) {
   smooth<float, float>(s, 0, s.p, s.rhs, 1, false, nullptr, nullptr, st);
@@ -1367,10 +1569,11 @@ void launch_residual_norm(const DevState& s, double* out, cudaStream_t st) {
 static void mixed_solve(const DevState& s, cudaStream_t st) {
   const size_t n = s.g.n();
   MixLv M[kMaxLevels];
-  M[0] = {s.e0, s.r0, nullptr, nullptr, false};
+  M[0] = {s.e0, s.r0, nullptr, nullptr, false, s.e0, nullptr};
   for (int l = 1; l < s.nlev; ++l) {
-    const bool h = l >= kMixedBF16Level;
-    M[l] = {h ? nullptr : s.lv[l].e, h ? nullptr : s.lv[l].b, h ? s.lv[l].eh : nullptr, h ? s.lv[l].bh : nullptr, h};
+    const bool h = l >= kMixedBF16Level, leg = leg_ok(s, l);
+    M[l] = {h ? nullptr : s.lv[l].e, h ? nullptr : s.lv[l].b, h ? s.lv[l].eh : nullptr, h ? s.lv[l].bh : nullptr, h,
+            h ? nullptr : (leg ? s.lv[l].e2 : s.lv[l].e), h ? (leg ? s.lv[l].eh2 : s.lv[l].eh) : nullptr};
   }
   unsigned int* done = s.redu + REDU_DONE;
   unsigned int* inner_done = s.redu + REDU_INNER_DONE;
@@ -1395,13 +1598,10 @@ static void mixed_solve(const DevState& s, cudaStream_t st) {
   };
   // the rest of the cycle: coarser levels and the level-0 post-smoothing
   auto tail = [&](cudaStream_t q, const unsigned int* skip) {
-    for (int l = 1; l < L - 1; ++l) {
-      mix_smooth(s, l, M, s.pre, true, false, skip, q);
-      mix_restrict(s, l, M, skip, q);
-    }
+    for (int l = 1; l < L - 1; ++l) mix_down(s, l, M, skip, q);
     if (M[L - 1].h) coarse_solve<__nv_bfloat16>(s, L - 1, M[L - 1].eh, M[L - 1].bh, skip, q);
     else coarse_solve<float>(s, L - 1, M[L - 1].ef, M[L - 1].bf, skip, q);
-    for (int l = L - 2; l >= 1; --l) mix_smooth(s, l, M, s.post, false, true, skip, q);
+    for (int l = L - 2; l >= 1; --l) mix_up(s, l, M, skip, q);
     mix_smooth(s, 0, M, s.post0, false, true, skip, q);
   };
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
