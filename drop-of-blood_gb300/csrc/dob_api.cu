@@ -205,11 +205,34 @@ static const int kStepOrder[] = {
     DOB_STAGE_CLEAR_SPLATS, DOB_STAGE_PARCEL_EMIT, DOB_STAGE_PARCEL_ADVECT, DOB_STAGE_CONC_PREDICT,
     DOB_STAGE_CONC_RESOLVE};
 
-static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float* stage_ms, bool stats_div) {
+// side (stream capture only): a second branch of the captured step for the
+// work that the velocity solve does not need: the clears (flags, splat
+// accumulators) beside the advection, the emission (reads the wave and the
+// parcels) beside the solve, and the parcel advection, which reads the
+// projected centre velocity and the dye, beside the dye predictor; it joins
+// before the resolve in reference mode, which reads the splats, and at the
+// step's end in the closed box.
+static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float* stage_ms, bool stats_div,
+                              cudaStream_t side = nullptr) {
   const int n = (int)(sizeof(kStepOrder) / sizeof(kStepOrder[0]));
+  auto order = [&](int ev, cudaStream_t first, cudaStream_t then) {  // `then` goes on after the work on `first`
+    cudaEventRecord(ctx->side_ev[ev], first);
+    cudaStreamWaitEvent(then, ctx->side_ev[ev], 0);
+  };
+  if (side) {
+    order(0, st, side);
+    launch_dye_flags_clear(s, side);
+    if (!s.ref) cudaMemsetAsync(s.redu + REDU_SPEED, 0, sizeof(unsigned int), side);
+    launch_clear_splats(s, side);
+  }
   // the wave substep comes first and the advection reads its result
   // (BloodDropEngine.ts:1886-1912)
   if (s.flags & DOB_PHYS_WAVE) launch_wave_step(s, st);
+  if (side) {
+    order(1, st, side);
+    launch_parcel_emit(s, side);
+    cudaEventRecord(ctx->side_ev[2], side);
+  }
   bool centre_fused = false;  // reference mode: the projection has formed the centre velocity
   for (int k = 0; k < n; ++k) {
     const int stage = kStepOrder[k];
@@ -218,13 +241,23 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
     // closed box: the centre after advection has no reader, and the centre
     // after the projection comes out of the fused projection kernel
     if (!s.ref && stage == DOB_STAGE_MAC_TO_CENTER) continue;
+    if (side && (stage == DOB_STAGE_CLEAR_SPLATS || stage == DOB_STAGE_PARCEL_EMIT)) continue;
+    if (side && stage == DOB_STAGE_PARCEL_ADVECT) {
+      order(1, st, side);
+      launch_parcel_advect(s, side);
+      cudaEventRecord(ctx->side_ev[3], side);
+      continue;
+    }
+    // the cleared flags, before the first kernel that writes them
+    if (side && stage == DOB_STAGE_PROJECT) cudaStreamWaitEvent(st, ctx->side_ev[2], 0);
+    if (side && s.ref && stage == DOB_STAGE_CONC_RESOLVE) cudaStreamWaitEvent(st, ctx->side_ev[3], 0);
     if (stage_ms) cudaEventRecord(ctx->stage_ev[0], st);
     if (!s.ref && stage == DOB_STAGE_PROJECT) {
       // with statistics the projection also forms max |div| (no separate
       // pass), and always the bound on the centre velocity that lets the
       // predictor skip blocks that cannot reach dye
       if (stats_div) cudaMemsetAsync(s.redu + REDU_MAXDIV, 0, sizeof(unsigned int), st);
-      cudaMemsetAsync(s.redu + REDU_SPEED, 0, sizeof(unsigned int), st);
+      if (!side) cudaMemsetAsync(s.redu + REDU_SPEED, 0, sizeof(unsigned int), st);
       launch_project_center_box(s, st, ctx->cfg.dt / ctx->cfg.dx, stats_div ? s.redu + REDU_MAXDIV : nullptr,
                                 s.redu + REDU_SPEED);
       swap_vel(s);
@@ -243,9 +276,14 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
     } else if (!s.ref && stage == DOB_STAGE_CONC_PREDICT) {
       // closed box: the predictor brackets its taps for the resolve, which
       // then traces only the forward sample; both skip clear water
-      launch_conc_predict(s, st, true, true);
+      launch_conc_predict(s, st, true, true, side != nullptr);
     } else if (!s.ref && stage == DOB_STAGE_CONC_RESOLVE) {
-      launch_dye_resolve_lim(s, st);
+      launch_dye_resolve_lim(s, st, side != nullptr);
+      std::swap(s.conc, s.conc2);
+    } else if (side && stage == DOB_STAGE_CONC_PREDICT) {
+      launch_conc_predict(s, st, false, true, true);
+    } else if (side && stage == DOB_STAGE_CONC_RESOLVE) {
+      launch_conc_resolve(s, st, true, true);
       std::swap(s.conc, s.conc2);
     } else {
       enqueue_stage(ctx, s, stage, st, true);
@@ -270,6 +308,7 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
       launch_divergence(s, nullptr, scale, s.redu + REDU_MAXDIV, st);
     }
   }
+  if (side && !s.ref) cudaStreamWaitEvent(st, ctx->side_ev[3], 0);
 }
 
 // Graphs are cached per (statistics on/off, dye and velocity buffers at the
@@ -304,7 +343,7 @@ static dob_status get_graph(dob_ctx* ctx, bool stats, bool injected, dob_ctx::St
   if (injected) s.cycles = ctx->cfg.mg_cycles_injected;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  enqueue_step_body(ctx, s, ctx->stream, nullptr, stats);
+  enqueue_step_body(ctx, s, ctx->stream, nullptr, stats, ctx->side_stream);
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   if (e != cudaSuccess) return fail(ctx, DOB_ECUDA, "cudaStreamEndCapture", cudaGetErrorString(e));
   size_t nn = 0;
@@ -490,6 +529,10 @@ dob_status dob_create(const dob_config* cfg, dob_ctx** out) {
   CK(cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&ctx->aux_stream, cudaStreamNonBlocking));
   CK(cudaStreamCreateWithFlags(&ctx->aux_stream2, cudaStreamNonBlocking));
+  int prio_low = 0, prio_high = 0;
+  CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
+  CK(cudaStreamCreateWithPriority(&ctx->side_stream, cudaStreamNonBlocking, prio_high));
+  for (cudaEvent_t& ev : ctx->side_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   CK(mg_prepare());
   s.aux = ctx->aux_stream;
   s.aux2 = ctx->aux_stream2;
@@ -635,6 +678,9 @@ void dob_destroy(dob_ctx* ctx) {
   if (ctx->stream) cudaStreamDestroy(ctx->stream);
   if (ctx->aux_stream) cudaStreamDestroy(ctx->aux_stream);
   if (ctx->aux_stream2) cudaStreamDestroy(ctx->aux_stream2);
+  if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
+  for (cudaEvent_t ev : ctx->side_ev)
+    if (ev) cudaEventDestroy(ev);
   delete ctx;
 }
 

@@ -40,6 +40,10 @@ struct dob_ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t aux_stream = nullptr;   // body capture of conditional graph nodes
   cudaStream_t aux_stream2 = nullptr;  // the same, one nesting level up
+  // second branch of a captured step (enqueue_step_body) and the events that
+  // fork and join it; used in stream capture only
+  cudaStream_t side_stream = nullptr;
+  cudaEvent_t side_ev[4] = {};
   std::string err;
   float U[128];
   dob::StepParams* host_params = nullptr;  // pinned ring

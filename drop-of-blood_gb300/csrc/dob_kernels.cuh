@@ -319,15 +319,19 @@ void launch_project_center_ref(const DevState& s, cudaStream_t st);
 // by the projection's s.redu[REDU_SPEED] in the closed box): skip the
 // blocks the dye-brick flags show to be clear water (same results).  The
 // resolves always maintain the flags of the dye buffer they write.
-void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket = false, bool sparse = false);
-void launch_dye_resolve_lim(const DevState& s, cudaStream_t st);
+// cleared: launch_dye_flags_clear has cleared the flags that the predictor
+// and the resolve of this step write (else they clear them themselves).
+void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket = false, bool sparse = false,
+                         bool cleared = false);
+void launch_dye_resolve_lim(const DevState& s, cudaStream_t st, bool cleared = false);
+void launch_dye_flags_clear(const DevState& s, cudaStream_t st);
 // dye written from outside the step (injection, field I/O, snapshots, the
 // tape): every brick of both dye buffers may hold dye until the next resolve
 void launch_dye_bricks_unknown(const DevState& s, cudaStream_t st);
 // zero the splat accumulators: only the bricks a splat has marked (the
 // others hold zeros already), then clear their marks
 void launch_clear_splats(const DevState& s, cudaStream_t st);
-void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse = false);
+void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse = false, bool cleared = false);
 // number of 8x8x8 dye bricks (one uint32 flag each)
 size_t dye_brick_count(const Grid& gc);
 

@@ -1040,9 +1040,15 @@ void launch_dye_bricks_unknown(const DevState& s, cudaStream_t st) {
 }
 size_t dye_brick_count(const Grid& gc) { return brick_grid(gc).n(); }
 
-void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket, bool sparse) {
+void launch_dye_flags_clear(const DevState& s, cudaStream_t st) {
+  const size_t nb = brick_grid(s.gc).n() * sizeof(uint32_t);
+  if (s.ref && s.pbrick) cudaMemsetAsync(s.pbrick, 0, nb, st);
+  if (uint32_t* cb = brick_flags_of(s, s.conc2)) cudaMemsetAsync(cb, 0, nb, st);
+}
+
+void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket, bool sparse, bool cleared) {
   uint32_t* pb = s.ref ? s.pbrick : nullptr;
-  if (pb) cudaMemsetAsync(pb, 0, brick_grid(s.gc).n() * sizeof(uint32_t), st);
+  if (pb && !cleared) cudaMemsetAsync(pb, 0, brick_grid(s.gc).n() * sizeof(uint32_t), st);
   const uint32_t* cb = sparse ? brick_flags_of(s, s.conc) : nullptr;
   DOB_VEL_DISPATCH(s.prec, {
     if (cb && s.ref) {
@@ -1061,9 +1067,9 @@ void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket, bool 
   });
 }
 
-void launch_dye_resolve_lim(const DevState& s, cudaStream_t st) {
+void launch_dye_resolve_lim(const DevState& s, cudaStream_t st, bool cleared) {
   uint32_t* cb = brick_flags_of(s, s.conc2);
-  if (cb) cudaMemsetAsync(cb, 0, brick_grid(s.gc).n() * sizeof(uint32_t), st);
+  if (cb && !cleared) cudaMemsetAsync(cb, 0, brick_grid(s.gc).n() * sizeof(uint32_t), st);
   DOB_VEL_DISPATCH(s.prec, {
     k_dye_resolve_lim<VS, DS><<<cell_grid(s.gc), cell_block(), 0, st>>>(
         s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const DS*)s.conc, (const DS*)s.pred,
@@ -1071,11 +1077,11 @@ void launch_dye_resolve_lim(const DevState& s, cudaStream_t st) {
   });
 }
 
-void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse) {
+void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse, bool cleared) {
   uint32_t* cb = brick_flags_of(s, s.conc2);
   // reference mode: the resolve rewrites its output's flags; the closed box's
   // tracing resolve does not, so its output's flags say "may hold dye"
-  if (cb) cudaMemsetAsync(cb, s.ref ? 0 : 1, brick_grid(s.gc).n() * sizeof(uint32_t), st);
+  if (cb && !cleared) cudaMemsetAsync(cb, s.ref ? 0 : 1, brick_grid(s.gc).n() * sizeof(uint32_t), st);
   DOB_VEL_DISPATCH(s.prec, {
     if (s.ref) {
       dim3 gr = cell_grid(s.gc);
