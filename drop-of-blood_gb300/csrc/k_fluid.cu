@@ -81,7 +81,9 @@ __global__ void k_init_vel(Grid g, const StepParams* __restrict__ Pp, VS* u, VS*
 // bound by the latency of their gathers: their register caps (5, 8 and 8
 // blocks of 256 per SM, a few spilled bytes) buy resident warps, measured
 // at 192x256x192: 336 -> 327, 150 -> 131 and 94 -> 86 us.
-template <class VS>
+// (REF: the forms without the packed interpolation; with the reference
+// mode's extra terms around it the kernel spills more and runs 2 % slower.)
+template <bool REF, class VS>
 __device__ __forceinline__ float sample_mac(const Grid& g, const VS* a, dob_v3 uvw, int comp) {
   // 0.5 / n is half the host-formed 1 / n (the same quotient: scaling by a
   // power of two commutes with rounding)
@@ -89,15 +91,14 @@ __device__ __forceinline__ float sample_mac(const Grid& g, const VS* a, dob_v3 u
   if (comp == 1) uvw.y = uvw.y - 0.5f * g.ry;
   if (comp == 2) uvw.z = uvw.z - 0.5f * g.rz;
   uvw = clamp3(uvw, 0.001f, 0.999f);
-  const Taps t = make_taps_in(g, uvw.x, uvw.y, uvw.z);
-  return lerp8(t, a);
+  return REF ? lerp8(make_taps_in(g, uvw.x, uvw.y, uvw.z), a) : lerp8_in(g, uvw.x, uvw.y, uvw.z, a);
 }
 // midpoint trace from the face centre uvwF, whose centre velocity is v0
-template <class V4>
+template <bool REF, class V4>
 __device__ __forceinline__ dob_v3 trace_back(const Grid& g, const V4* cen, dob_v3 uvwF, dob_v3 v0, float dtv,
                                              const Recip3& dom) {
-  const dob_v3 uvwMid = clamp3(uvwF - (0.5f * (v0 * dtv)) / dom, 0.002f, 0.998f);
-  const dob_v3 vMid = sample_center_in(g, cen, uvwMid);
+  const dob_v3 uvwMid = clamp3(uvwF - (v0 * (0.5f * dtv)) / dom, 0.002f, 0.998f);  // 0.5 (v0 dt): exact scaling
+  const dob_v3 vMid = REF ? sample_center_in(g, cen, uvwMid) : sample_center_fast(g, cen, uvwMid);
   return clamp3(uvwF - (vMid * dtv) / dom, 0.002f, 0.998f);
 }
 __device__ __forceinline__ float azim_neck(float theta, float seed) {
@@ -105,8 +106,15 @@ __device__ __forceinline__ float azim_neck(float theta, float seed) {
          0.018f * dob_sin(8.0f * theta + seed * 0.89f);
 }
 
-template <class VS>
-__global__ void __launch_bounds__(256, 5) k_advect_mac(Grid g, const StepParams* __restrict__ Pp, int ref, int flags,
+// The closed box (REF = false, without the reference's terms) interpolates
+// pairs and clamps no tap away from the edges: 948 -> 860 instructions per 32
+// cells, 290 -> 280 us at 192x256x192, 804 -> 737 at 256x384x256; what is
+// left waits for the taps (4.5 L1 wavefronts per 16-byte load of a warp).
+// Four and six blocks per SM: 300 and 306 us; one face per thread (the three
+// faces' taps then miss L1): 457-540; blocks of 16x4x4, 32x4x2, 8x8x4: 286,
+// 278, 324.
+template <class VS, bool REF>
+__global__ void __launch_bounds__(256, 5) k_advect_mac(Grid g, const StepParams* __restrict__ Pp, int flags,
                                                     const VS* __restrict__ u, const VS* __restrict__ v,
                                                     const VS* __restrict__ w,
                                                     const typename Vec4Of<VS>::type* __restrict__ cen,
@@ -131,10 +139,10 @@ __global__ void __launch_bounds__(256, 5) k_advect_mac(Grid g, const StepParams*
   const dob_v3 v0X = bx && ay && az ? face_mean(cen, i, 1) : sample_center_exact(g, cen, v3(cb.x, ca.y, ca.z));
   const dob_v3 v0Y = ax && by && az ? face_mean(cen, i, sy) : sample_center_exact(g, cen, v3(ca.x, cb.y, ca.z));
   const dob_v3 v0Z = ax && ay && bz ? face_mean(cen, i, sz) : sample_center_exact(g, cen, v3(ca.x, ca.y, cb.z));
-  float vx = sample_mac(g, u, trace_back(g, cen, uvwX, v0X, dtv, dom), 0) * damp;
-  float vy = sample_mac(g, v, trace_back(g, cen, uvwY, v0Y, dtv, dom), 1) * damp;
-  float vz = sample_mac(g, w, trace_back(g, cen, uvwZ, v0Z, dtv, dom), 2) * damp;
-  if (ref) {
+  float vx = sample_mac<REF>(g, u, trace_back<REF>(g, cen, uvwX, v0X, dtv, dom), 0) * damp;
+  float vy = sample_mac<REF>(g, v, trace_back<REF>(g, cen, uvwY, v0Y, dtv, dom), 1) * damp;
+  float vz = sample_mac<REF>(g, w, trace_back<REF>(g, cen, uvwZ, v0Z, dtv, dom), 2) * damp;
+  if (REF) {
     const float surfY = P.U[40];
     const dob_v3 pCell = to_world(P, (v3((float)x, (float)y, (float)z) + v3(0.5f, 0.5f, 0.5f)) / dimr);
     const dob_v3 pFaceY = to_world(P, uvwY);
@@ -239,7 +247,7 @@ __global__ void __launch_bounds__(256, 5) k_advect_mac(Grid g, const StepParams*
   }
   if (x >= g.nx - 1) vx = 0.0f;
   if (z >= g.nz - 1) vz = 0.0f;
-  if (!ref && y >= g.ny - 1) vy = 0.0f;
+  if (!REF && y >= g.ny - 1) vy = 0.0f;
   stf(uo + i, vx); stf(vo + i, vy); stf(wo + i, vz);
 }
 
@@ -322,7 +330,7 @@ __device__ __forceinline__ dob_v3 vort_conf(const Grid& g, const V4* curl, int i
 template <class DS>
 __device__ __forceinline__ dob_v3 sample_conc_rg(const Grid& gc, const typename Vec4Of<DS>::type* conc4, dob_v3 uvw) {
   const Taps t = make_taps(gc, uvw.x, uvw.y, uvw.z);
-  const float4 r = lerp8x4(t, conc4);
+  const float4 r = lerp8xn<2>(t, conc4);
   return v3(r.x, r.y, 0.0f);
 }
 
@@ -630,7 +638,7 @@ __device__ __forceinline__ void predict_cell(const Grid& gc, const Grid& g, cons
       back = clamp3(uvw - (vMid * dtv) / dom, 0.001f, 0.999f);
     }
     const Taps t = make_taps_in(gc, back.x, back.y, back.z);
-    const float pv = lerp8x4(t, conc4).y;
+    const float pv = lerp8xn<2>(t, conc4).y;
     stf(pred + i, pv);
     if (pbrick && pv != 0.0f) mark_brick(gc, pbrick, x, y, z);
   } else {
@@ -965,9 +973,13 @@ void launch_init_vel(const DevState& s, cudaStream_t st) {
 
 void launch_advect_mac(const DevState& s, cudaStream_t st) {
   DOB_VEL_DISPATCH(s.prec, {
-    k_advect_mac<VS><<<cell_grid(s.g), cell_block(), 0, st>>>(
-        s.g, s.params, s.ref, s.flags, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w,
-        (const typename Vec4Of<VS>::type*)s.cen, s.wave, (VS*)s.u2, (VS*)s.v2, (VS*)s.w2);
+    auto run = [&](auto* k) {
+      k<<<cell_grid(s.g), cell_block(), 0, st>>>(s.g, s.params, s.flags, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w,
+                                                 (const typename Vec4Of<VS>::type*)s.cen, s.wave, (VS*)s.u2, (VS*)s.v2,
+                                                 (VS*)s.w2);
+    };
+    if (s.ref) run(k_advect_mac<VS, true>);
+    else run(k_advect_mac<VS, false>);
   });
 }
 
