@@ -105,9 +105,8 @@ struct AdjState {
   float4* acen;            // adjoint of the centre velocity (x, y, z, unused)
   float *ac, *ac2, *apred; // dye (input), resolved dye (output), predictor
   float *ap, *arhs;        // pressure, right-hand side (split)
-  float* le[kMaxLevels];   // coarse corrections (split, levels >= 1)
-  float* lb[kMaxLevels];   // coarse right-hand sides (split, levels >= 1)
-  float *alpha, *gq;       // Casson adjoint scratch: per-cell alpha, 2 dL/dQ
+  float* lr[kMaxLevels];   // residuals of the transposed cycle (split, levels >= 1)
+  float *alpha, *gq;       // Casson adjoint scratch: per-cell alpha, 2 dL/dQ (and the transposed cycle's)
   double* part;            // partial sums of the mean removals: 2 x kSumBlocks
   float *lam, *lamlo;      // mixed mode: adjoint pressure solve's solution pair (split)
   double* red;             // FP64 reduction slots (mean removal)
@@ -356,6 +355,12 @@ cudaError_t mg_prepare();
 // (it then needs its second array, MgLevel::e2 / eh2).
 bool mg_leg_level(const Grid& d);
 void launch_pressure_solve(const DevState& s, cudaStream_t st);
+// Transpose of its FP32 V-cycles (all s.cycles of them): ap, the adjoint of
+// the pressure, is replaced by the adjoint of the warm start, arhs gains the
+// right-hand side's.  x0, t0: scratch of the finest grid's size, R[l] of
+// every level l >= 1.
+void launch_transposed_cycles(const DevState& s, float* ap, float* arhs, float* x0, float* t0, float* const* R,
+                              cudaStream_t st);
 void launch_residual_norm(const DevState& s, double* out, cudaStream_t st);
 // mean removal: launch_sum leaves per-block partials in part (kSumBlocks
 // doubles), launch_sub_mean adds them in a fixed order and subtracts the mean
@@ -396,7 +401,5 @@ void launch_adj_pressure_solve(const DevState& s, const AdjState& a, cudaStream_
 void launch_adj_project(const DevState& s, const AdjState& a, cudaStream_t st);
 void launch_adj_conc_predict(const DevState& s, const AdjState& a, cudaStream_t st);
 void launch_adj_conc_resolve(const DevState& s, const AdjState& a, cudaStream_t st);
-// Raise the dynamic shared-memory limit of the transposed coarse solve.
-cudaError_t adj_prepare();
 
 }  // namespace dob

@@ -183,11 +183,16 @@ __device__ __forceinline__ void leg_store(const Grid& d, const LegCol<L>& t, con
 // zero; else the preceding launch was the first red half-sweep on a, whose red
 // cells are read, and the loads of b, which it did not write, issue ahead of
 // the wait for it.
-template <class T, class TC, class L, bool ZERO>
+// TR (with ZERO; the transposed cycle): the colours change places, and the
+// residual of the black cells goes to res (the red ones, updated last, have
+// none but rounding).
+template <class T, class TC, class L, bool ZERO, bool TR>
 __global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, float inv_h2, int ref,
                                                     const T* __restrict__ a, const T* __restrict__ b,
-                                                    T* __restrict__ out, TC* __restrict__ bc,
+                                                    T* __restrict__ out, TC* __restrict__ bc, T* __restrict__ res,
                                                     const unsigned int* __restrict__ skip) {
+  static_assert(ZERO || !TR, "the transposed cycle starts from zero");
+  constexpr int c0 = TR ? 1 : 0;  // the colour of the first half-sweep
   __shared__ LegShared<L> sh;
   const LegCol<L> t(d, ref);
   float e[2][kLegZ], bb[2][kLegZ];
@@ -202,36 +207,44 @@ __global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, f
     leg_load<T, L>(d, t, b, 0, bb[0]);
     leg_load<T, L>(d, t, b, 1, bb[1]);
 #pragma unroll
-    for (int i = 0; i < kLegZ; ++i) e[0][i] = leg_value<T, L>(d, t, 0, i, 0.0f - h2 * bb[0][i]);
+    for (int i = 0; i < kLegZ; ++i) e[c0][i] = leg_value<T, L>(d, t, c0, i, 0.0f - h2 * bb[c0][i]);
   } else {
-    leg_load<T, L>(d, t, a, 0, e[0]);
+    leg_load<T, L>(d, t, a, c0, e[c0]);
   }
-  leg_share<L>(sh, t, 0, e[0]);
+  leg_share<L>(sh, t, c0, e[c0]);
   __syncthreads();
   if constexpr (L::S == 2) {
-    leg_half<T, L, 3>(d, h2, t, sh, 1, e, bb);
-    leg_half<T, L, 2>(d, h2, t, sh, 0, e, bb);
+    leg_half<T, L, 3>(d, h2, t, sh, 1 - c0, e, bb);
+    leg_half<T, L, 2>(d, h2, t, sh, c0, e, bb);
   }
-  leg_half<T, L, 1>(d, h2, t, sh, 1, e, bb);
+  leg_half<T, L, 1>(d, h2, t, sh, 1 - c0, e, bb);
   leg_store<T, L>(d, t, e, out);
+  auto residual = [&](int c, int i) {
+    const float sumN = leg_sum<L>(t, sh, e, c, i);
+    const bool w = t.wall_z(d, i), p = t.par(c, i) != 0;
+    const float dg = w ? (p ? t.d1[1] : t.d1[0]) : (p ? t.d0[1] : t.d0[0]);
+    const float lap = (sumN - dg * e[c][i]) * inv_h2;
+    return bb[c][i] - lap;
+  };
+  const bool mine = t.in && t.kk >= L::H / 2 && t.kk < L::H / 2 + L::TX / 2 && t.yy >= L::H && t.yy < L::H + L::TY;
+  if constexpr (TR) {
+    T* r = res + (uint32_t)(d.n() >> 1);
+#pragma unroll
+    for (int i = L::H; i < kLegZ; ++i) {
+      const float v = residual(1, i);
+      if (mine && t.has_z(d, i)) stf(r + t.off(i), v);
+    }
+    return;
+  }
   // the residuals of a coarse cell: x = 2k, 2k + 1 and both planes are this
   // thread's, the row above the next row's thread's
-  const bool put = t.in && t.kk >= L::H / 2 && t.kk < L::H / 2 + L::TX / 2 && t.yy >= L::H && t.yy < L::H + L::TY &&
-                   (t.yy & 1) == 0;
+  const bool put = mine && (t.yy & 1) == 0;
 #pragma unroll
   for (int i = L::H; i < kLegZ; i += 2) {
     float r[2][2], u[2][2];  // [index][x] of this row and the next
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      float rc[2];
-#pragma unroll
-      for (int c = 0; c < 2; ++c) {
-        const float sumN = leg_sum<L>(t, sh, e, c, i + j);
-        const bool w = t.wall_z(d, i + j), p = t.par(c, i + j) != 0;
-        const float dg = w ? (p ? t.d1[1] : t.d1[0]) : (p ? t.d0[1] : t.d0[0]);
-        const float lap = (sumN - dg * e[c][i + j]) * inv_h2;
-        rc[c] = bb[c][i + j] - lap;
-      }
+      const float rc[2] = {residual(0, i + j), residual(1, i + j)};
       const bool sw = t.par(0, i + j) != 0;  // colour 0's cell is x = 2k + 1
       r[j][0] = sw ? rc[1] : rc[0];
       r[j][1] = sw ? rc[0] : rc[1];
@@ -254,81 +267,102 @@ __global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, f
 // into out.  Only the black cells take the correction (the first half-sweep
 // overwrites the red ones without reading them).  a and b were not written
 // by the preceding launch: their loads issue ahead of the wait for it.
-template <class T, class TC, class L>
+// TR (the transposed cycle): the colours change places, and the correction is
+// an eighth of ec's cell (the transpose of the restriction's average).
+template <class T, class TC, class L, bool TR>
 __global__ void __launch_bounds__(L::NT) k_leg_up(Grid d, Grid dc, float h2, int ref, const T* __restrict__ a,
                                                   const T* __restrict__ b, const TC* __restrict__ ec,
                                                   T* __restrict__ out, const unsigned int* __restrict__ skip) {
   __shared__ LegShared<L> sh;
-  __shared__ float C[L::CZ][L::CY][L::CX];  // coarse taps, clamped at the grid (0 above a Dirichlet top)
+  // coarse taps, clamped at the grid (0 above a Dirichlet top)
+  __shared__ float C[TR ? 1 : L::CZ][L::CY][L::CX];
   const LegCol<L> t(d, ref);
   float e[2][kLegZ], bb[2][kLegZ];
   leg_load<T, L>(d, t, b, 0, bb[0]);
   leg_load<T, L>(d, t, b, 1, bb[1]);
-  leg_load<T, L>(d, t, a, 1, e[1]);
-  // first coarse tap: the region's corner is even, so fine cell i of an axis
-  // interpolates taps (i + 1) / 2 and (i + 1) / 2 + 1
-  const int Z0 = (int)blockIdx.z * L::TZ - L::H;
-  const int XC = t.k - t.kk - 1, YC = ((int)blockIdx.y * L::TY - L::H) / 2 - 1, ZC = Z0 / 2 - 1;
-  auto frac = [](int i, int n, float r, int m) {
-    const float u = __fmaf_rn(div_by((float)i + 0.5f, (float)n, r), (float)m, -0.5f);
-    return u - floorf(u);
-  };
-  const float fx0 = frac(2 * t.k, d.nx, d.rx, dc.nx), fx1 = frac(2 * t.k + 1, d.nx, d.rx, dc.nx);
-  const float fy = frac(t.y, d.ny, d.ry, dc.ny);
-  pdl_wait();
-  pdl_trigger();
-  if (skip_now(skip)) return;
+  constexpr int c0 = TR ? 0 : 1;  // the colour that takes the correction
+  leg_load<T, L>(d, t, a, c0, e[c0]);
+  if constexpr (TR) {
+    pdl_wait();
+    pdl_trigger();
+    if (skip_now(skip)) return;
+    const uint32_t hc = (uint32_t)(dc.nx >> 1), halfc = (uint32_t)(dc.n() >> 1);
 #pragma unroll
-  for (int i0 = 0; i0 < L::CX * L::CY * L::CZ; i0 += L::NT) {
-    const int i = i0 + (int)threadIdx.x;
-    if (i < L::CX * L::CY * L::CZ) {
-      const int xi = i % L::CX, yi = (i / L::CX) % L::CY, zi = i / (L::CX * L::CY);
-      const int X = dob_clampi(XC + xi, 0, dc.nx - 1), Y = dob_clampi(YC + yi, 0, dc.ny - 1),
-                Z = dob_clampi(ZC + zi, 0, dc.nz - 1);
-      const uint32_t j = (((X + Y + Z) & 1) ? (uint32_t)(dc.n() >> 1) : 0u) +
-                         ((uint32_t)Z * dc.ny + (uint32_t)Y) * (uint32_t)(dc.nx >> 1) + (uint32_t)(X >> 1);
-      const float v = ldv(ec + j);
-      C[zi][yi][xi] = ref && YC + yi >= dc.ny ? 0.0f : v;
+    for (int i = 0; i < kLegZ; i += 2) {  // planes i and i + 1 have one parent
+      const int Y = t.y >> 1, Z = t.z(i) >> 1;
+      const bool on = t.in && t.has_z(d, i);
+      const float v =
+          on ? 0.125f * ldv(ec + ((((t.k + Y + Z) & 1) ? halfc : 0u) + ((uint32_t)Z * dc.ny + Y) * hc + (t.k >> 1)))
+             : 0.0f;
+      e[c0][i] = on ? as_stored<T>(e[c0][i] + v) : 0.0f;
+      e[c0][i + 1] = on ? as_stored<T>(e[c0][i + 1] + v) : 0.0f;
+    }
+  } else {
+    // first coarse tap: the region's corner is even, so fine cell i of an axis
+    // interpolates taps (i + 1) / 2 and (i + 1) / 2 + 1
+    const int Z0 = (int)blockIdx.z * L::TZ - L::H;
+    const int XC = t.k - t.kk - 1, YC = ((int)blockIdx.y * L::TY - L::H) / 2 - 1, ZC = Z0 / 2 - 1;
+    auto frac = [](int i, int n, float r, int m) {
+      const float u = __fmaf_rn(div_by((float)i + 0.5f, (float)n, r), (float)m, -0.5f);
+      return u - floorf(u);
+    };
+    const float fx0 = frac(2 * t.k, d.nx, d.rx, dc.nx), fx1 = frac(2 * t.k + 1, d.nx, d.rx, dc.nx);
+    const float fy = frac(t.y, d.ny, d.ry, dc.ny);
+    pdl_wait();
+    pdl_trigger();
+    if (skip_now(skip)) return;
+#pragma unroll
+    for (int i0 = 0; i0 < L::CX * L::CY * L::CZ; i0 += L::NT) {
+      const int i = i0 + (int)threadIdx.x;
+      if (i < L::CX * L::CY * L::CZ) {
+        const int xi = i % L::CX, yi = (i / L::CX) % L::CY, zi = i / (L::CX * L::CY);
+        const int X = dob_clampi(XC + xi, 0, dc.nx - 1), Y = dob_clampi(YC + yi, 0, dc.ny - 1),
+                  Z = dob_clampi(ZC + zi, 0, dc.nz - 1);
+        const uint32_t j = (((X + Y + Z) & 1) ? (uint32_t)(dc.n() >> 1) : 0u) +
+                           ((uint32_t)Z * dc.ny + (uint32_t)Y) * (uint32_t)(dc.nx >> 1) + (uint32_t)(X >> 1);
+        const float v = ldv(ec + j);
+        C[zi][yi][xi] = ref && YC + yi >= dc.ny ? 0.0f : v;
+      }
+    }
+    __syncthreads();
+    // coarse plane m interpolated in x and y at this row's cells x = 2k (s0)
+    // and 2k + 1 (s1); region plane zz interpolates coarse planes (zz + 1) / 2
+    // and the next: going inwards from index 0, the lower half meets planes
+    // 0, 1, .. with (zz + 1) / 2 = (i + 1) / 2, the upper half planes 9, 8, ..
+    // with (zz + 1) / 2 + 1 = 9 - (i + 1) / 2
+    auto plane = [&](int m, float& s0, float& s1) {
+      const float* c0 = &C[t.up ? L::CZ - 1 - m : m][(t.yy + 1) >> 1][t.kk];
+      const float* c1 = c0 + L::CX;
+      s0 = dob_mix(dob_mix(c0[0], c0[1], fx0), dob_mix(c1[0], c1[1], fx0), fy);
+      s1 = dob_mix(dob_mix(c0[1], c0[2], fx1), dob_mix(c1[1], c1[2], fx1), fy);
+    };
+    float lo0, lo1;
+    plane(0, lo0, lo1);
+#pragma unroll
+    for (int m = 0; m <= kLegZ / 2; ++m) {
+      float hi0, hi1;
+      plane(m + 1, hi0, hi1);
+#pragma unroll
+      for (int i = 2 * m - 1; i <= 2 * m; ++i) {
+        if (i < 0 || i >= kLegZ) continue;
+        const bool p = t.par(1, i) != 0;
+        const float fz = frac(t.z(i), d.nz, d.rz, dc.nz);
+        const float u = p ? lo1 : lo0, v = p ? hi1 : hi0;  // the outer and the inner plane
+        const float corr = dob_mix(t.up ? v : u, t.up ? u : v, fz);
+        e[1][i] = t.in && t.has_z(d, i) ? as_stored<T>(e[1][i] + corr) : 0.0f;
+      }
+      lo0 = hi0;
+      lo1 = hi1;
     }
   }
-  __syncthreads();
-  // coarse plane m interpolated in x and y at this row's cells x = 2k (s0)
-  // and 2k + 1 (s1); region plane zz interpolates coarse planes (zz + 1) / 2
-  // and the next: going inwards from index 0, the lower half meets planes
-  // 0, 1, .. with (zz + 1) / 2 = (i + 1) / 2, the upper half planes 9, 8, ..
-  // with (zz + 1) / 2 + 1 = 9 - (i + 1) / 2
-  auto plane = [&](int m, float& s0, float& s1) {
-    const float* c0 = &C[t.up ? L::CZ - 1 - m : m][(t.yy + 1) >> 1][t.kk];
-    const float* c1 = c0 + L::CX;
-    s0 = dob_mix(dob_mix(c0[0], c0[1], fx0), dob_mix(c1[0], c1[1], fx0), fy);
-    s1 = dob_mix(dob_mix(c0[1], c0[2], fx1), dob_mix(c1[1], c1[2], fx1), fy);
-  };
-  float lo0, lo1;
-  plane(0, lo0, lo1);
-#pragma unroll
-  for (int m = 0; m <= kLegZ / 2; ++m) {
-    float hi0, hi1;
-    plane(m + 1, hi0, hi1);
-#pragma unroll
-    for (int i = 2 * m - 1; i <= 2 * m; ++i) {
-      if (i < 0 || i >= kLegZ) continue;
-      const bool p = t.par(1, i) != 0;
-      const float fz = frac(t.z(i), d.nz, d.rz, dc.nz);
-      const float u = p ? lo1 : lo0, v = p ? hi1 : hi0;  // the outer and the inner plane
-      const float corr = dob_mix(t.up ? v : u, t.up ? u : v, fz);
-      e[1][i] = t.in && t.has_z(d, i) ? as_stored<T>(e[1][i] + corr) : 0.0f;
-    }
-    lo0 = hi0;
-    lo1 = hi1;
-  }
-  leg_share<L>(sh, t, 1, e[1]);
+  leg_share<L>(sh, t, c0, e[c0]);
   __syncthreads();
   if constexpr (L::S == 2) {
-    leg_half<T, L, 3>(d, h2, t, sh, 0, e, bb);
-    leg_half<T, L, 2>(d, h2, t, sh, 1, e, bb);
+    leg_half<T, L, 3>(d, h2, t, sh, 1 - c0, e, bb);
+    leg_half<T, L, 2>(d, h2, t, sh, c0, e, bb);
   }
-  leg_half<T, L, 1>(d, h2, t, sh, 0, e, bb);
-  leg_half<T, L, 0>(d, h2, t, sh, 1, e, bb);
+  leg_half<T, L, 1>(d, h2, t, sh, 1 - c0, e, bb);
+  leg_half<T, L, 0>(d, h2, t, sh, c0, e, bb);
   leg_store<T, L>(d, t, e, out);
 }
 

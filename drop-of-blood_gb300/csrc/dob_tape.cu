@@ -118,8 +118,6 @@ dob_status alloc(dob_ctx* ctx, std::vector<void*>& list, void** p, size_t bytes)
 // Adjoint arrays, allocated (zeroed) on first use.
 dob_status ensure_adj(dob_ctx* ctx) {
   if (ctx->adj) return DOB_OK;
-  cudaError_t pe = adj_prepare();
-  if (pe != cudaSuccess) return record_error(ctx, DOB_ECUDA, "adj_prepare", cudaGetErrorString(pe));
   AdjCtx* A = new AdjCtx();
   memset(&A->a, 0, sizeof(A->a));
   ctx->adj = A;
@@ -135,10 +133,8 @@ dob_status ensure_adj(dob_ctx* ctx) {
   F(&a.ac, Nc); F(&a.ac2, Nc); F(&a.apred, Nc);
   F(&a.ap, N); F(&a.arhs, N); F(&a.alpha, N); F(&a.gq, N);
   if (s.prec == DOB_PREC_MIXED) { F(&a.lam, N); F(&a.lamlo, N); }
-  for (int l = 1; l < s.nlev; ++l) {
-    F(&a.le[l], s.lv[l].d.n());
-    F(&a.lb[l], s.lv[l].d.n());
-  }
+  if (s.prec != DOB_PREC_MIXED)
+    for (int l = 1; l < s.nlev; ++l) F(&a.lr[l], s.lv[l].d.n());
   if (st == DOB_OK) st = alloc(ctx, A->bufs, (void**)&a.red, 8 * sizeof(double));
   if (st == DOB_OK) st = alloc(ctx, A->bufs, (void**)&a.part, 2 * kSumBlocks * sizeof(double));
   if (st == DOB_OK) st = alloc(ctx, A->bufs, (void**)&A->dred, 4 * sizeof(double));
@@ -154,10 +150,6 @@ void zero_adj(const DevState& s, const AdjState& a, cudaStream_t st) {
   if (a.lam) {  // mixed mode: the adjoint pressure solve's warm start
     cudaMemsetAsync(a.lam, 0, N * 4, st);
     cudaMemsetAsync(a.lamlo, 0, N * 4, st);
-  }
-  for (int l = 1; l < s.nlev; ++l) {
-    cudaMemsetAsync(a.le[l], 0, s.lv[l].d.n() * 4, st);
-    cudaMemsetAsync(a.lb[l], 0, s.lv[l].d.n() * 4, st);
   }
 }
 

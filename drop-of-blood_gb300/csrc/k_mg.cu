@@ -538,6 +538,159 @@ __global__ void __launch_bounds__(256, ZC == 4 ? 3 : 4) k_prolong_add2(Grid f, G
   }
 }
 
+// ---- the transposed cycle's transfers and residuals (FP32) -------------------------------
+// Weight of coarse index J in the interpolation at fine index xf (the
+// prolongation's clamped taps; 0 above a Dirichlet top when `top0`); rnf = 1/nf.
+__device__ __forceinline__ float prolong_weight(int xf, int nf, float rnf, int nc, int J, bool top0) {
+  const float cx = __fmaf_rn(div_by((float)xf + 0.5f, (float)nf, rnf), (float)nc, -0.5f);  // as k_prolong_add2 forms it
+  const float bx = floorf(cx);
+  const float fx = cx - bx;
+  const int i0 = (int)bx, i1 = i0 + 1;
+  float w = 0.0f;
+  if (dob_clampi(i0, 0, nc - 1) == J && !(top0 && i0 >= nc)) w += 1.0f - fx;
+  if (dob_clampi(i1, 0, nc - 1) == J && !(top0 && i1 >= nc)) w += fx;
+  return w;
+}
+// Transpose of k_prolong_add2: bc(X) = sum of the interpolation weight on X
+// times r over the fine cells 2X-1..2X+2 of each axis, two coarse cells per
+// thread.  BLACK: the red cells of r count as zero and are not read.
+template <bool BLACK>
+__global__ void __launch_bounds__(256) k_prolong_t2(Grid f, Grid c, int ref, const float* __restrict__ r,
+                                                    float* __restrict__ bc) {
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;
+  const int Y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int Z = blockIdx.z;
+  const bool inside = 2 * q < c.nx && Y < c.ny;
+  float wx0[4], wx1[4], wy[4], wz[4];
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const int x0 = 4 * q - 1 + a, x1 = 4 * q + 1 + a;
+    wx0[a] = (x0 >= 0 && x0 < f.nx) ? prolong_weight(x0, f.nx, f.rx, c.nx, 2 * q, false) : 0.0f;
+    wx1[a] = (x1 >= 0 && x1 < f.nx) ? prolong_weight(x1, f.nx, f.rx, c.nx, 2 * q + 1, false) : 0.0f;
+    const int yf = 2 * Y - 1 + a, zf = 2 * Z - 1 + a;
+    wy[a] = (yf >= 0 && yf < f.ny) ? prolong_weight(yf, f.ny, f.ry, c.ny, Y, ref != 0) : 0.0f;
+    wz[a] = (zf >= 0 && zf < f.nz) ? prolong_weight(zf, f.nz, f.rz, c.nz, Z, false) : 0.0f;
+  }
+  pdl_wait();
+  pdl_trigger();
+  if (!inside) return;
+  const uint32_t hx = (uint32_t)f.nx >> 1, half = (uint32_t)(f.n() >> 1), sz = (uint32_t)f.ny * hx;
+  const uint32_t w = 2u * (uint32_t)q;
+  const bool has_lo = q > 0, has_hi = 4 * q + 4 < f.nx;
+  float acc0 = 0.0f, acc1 = 0.0f;
+#pragma unroll
+  for (int cz = 0; cz < 4; ++cz) {
+    if (wz[cz] == 0.0f) continue;
+#pragma unroll
+    for (int by = 0; by < 4; ++by) {
+      if (wy[by] == 0.0f) continue;
+      const int yf = 2 * Y - 1 + by, zf = 2 * Z - 1 + cz, par = (yf + zf) & 1;
+      const uint32_t row = (uint32_t)zf * sz + (uint32_t)yf * hx + w;
+      const float* pe = r + (par ? half : 0u) + row;  // even cells 4q, 4q+2 (words 2q, 2q+1)
+      const float* po = r + (par ? 0u : half) + row;  // odd cells 4q+1, 4q+3
+      const float2 z2 = make_float2(0.0f, 0.0f);
+      // the even cells are black in rows of odd parity, the odd cells in the others
+      const float2 e = (!BLACK || par) ? Pair<float>::ld(pe) : z2, o = (!BLACK || !par) ? Pair<float>::ld(po) : z2;
+      const float lo = (has_lo && (!BLACK || !par)) ? po[-1] : 0.0f;  // x = 4q-1 (odd, word 2q-1)
+      const float hi = (has_hi && (!BLACK || par)) ? pe[2] : 0.0f;    // x = 4q+4 (even, word 2q+2)
+      const float v[6] = {lo, e.x, o.x, e.y, o.y, hi};
+      const float s0 = wx0[0] * v[0] + wx0[1] * v[1] + wx0[2] * v[2] + wx0[3] * v[3];
+      const float s1 = wx1[0] * v[2] + wx1[1] * v[3] + wx1[2] * v[4] + wx1[3] * v[5];
+      const float wyz = wy[by] * wz[cz];
+      acc0 = fmaf(wyz, s0, acc0);
+      acc1 = fmaf(wyz, s1, acc1);
+    }
+  }
+  const uint32_t hc = (uint32_t)c.nx >> 1, halfc = (uint32_t)(c.n() >> 1);
+  const uint32_t rc = ((uint32_t)Z * c.ny + Y) * hc + (uint32_t)q;
+  const int pc = (Y + Z) & 1;
+  bc[(pc ? halfc : 0u) + rc] = acc0;
+  bc[(pc ? 0u : halfc) + rc] = acc1;
+}
+// Transpose of the restriction's average: a += ec / 8 on the red cells (RED:
+// a black half-sweep follows and overwrites the others) or all of them, four
+// fine cells of one coarse row per thread.
+template <bool RED>
+__global__ void __launch_bounds__(256) k_inject_t2(Grid f, Grid c, float* __restrict__ a, const float* __restrict__ ec) {
+  pdl_wait();
+  pdl_trigger();
+  const int q = blockIdx.x * blockDim.x + threadIdx.x;  // coarse cells 2q, 2q + 1
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;  // fine row
+  const int z = blockIdx.z;
+  if (2 * q >= c.nx || y >= f.ny) return;
+  const uint32_t hc = (uint32_t)c.nx >> 1, halfc = (uint32_t)(c.n() >> 1);
+  const uint32_t rc = ((uint32_t)(z >> 1) * c.ny + (uint32_t)(y >> 1)) * hc + (uint32_t)q;
+  const int pc = ((y >> 1) + (z >> 1)) & 1;  // colour of coarse X = 2q
+  const float v0 = 0.125f * ec[(pc ? halfc : 0u) + rc], v1 = 0.125f * ec[(pc ? 0u : halfc) + rc];
+  const uint32_t hx = (uint32_t)f.nx >> 1, half = (uint32_t)(f.n() >> 1);
+  // words 2q and 2q + 1 of either colour are children of 2q and 2q + 1
+  float* p = a + ((uint32_t)z * f.ny + (uint32_t)y) * hx + 2u * (uint32_t)q;
+#pragma unroll
+  for (int k = 0; k < (RED ? 1 : 2); ++k) {
+    const float2 o = Pair<float>::ld(p + k * half);
+    Pair<float>::st(p + k * half, make_float2(o.x + v0, o.y + v1));
+  }
+}
+// r = b - A x: on the black cells into r (blockIdx.z = plane), or, TAKE, on
+// all cells into b itself with sum += x (blockIdx.z = 2 plane + colour).
+// Four cells of a row per thread as in k_rbgs_v4 (rows with nx % 8 == 0), or
+// one (VEC = 1).
+template <bool TAKE, int VEC>
+__global__ void __launch_bounds__(256) k_residual_t(Grid d, float inv_h2, int ref, const float* __restrict__ x,
+                                                    const float* b, float* r, float* __restrict__ sum) {
+  pdl_wait();
+  pdl_trigger();
+  const uint32_t hx = (uint32_t)d.nx >> 1, half = (uint32_t)(d.n() >> 1), sz = (uint32_t)d.ny * hx;
+  const uint32_t k0 = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int z = TAKE ? blockIdx.z >> 1 : blockIdx.z, color = TAKE ? blockIdx.z & 1 : 1;
+  if (k0 >= hx || y >= d.ny) return;
+  const uint32_t own = color ? half : 0u, oth = color ? 0u : half;
+  const uint32_t i = (uint32_t)z * sz + (uint32_t)y * hx + k0;
+  const bool has_ym = y > 0, has_yp = y < d.ny - 1, has_zm = z > 0, has_zp = z < d.nz - 1;
+  const int p = (y + z + color) & 1;
+  const bool has_e = p == 0 ? k0 > 0 : k0 + VEC < hx;  // the word before (p = 0) or after the others
+  const float dyz = (has_ym ? 1.0f : 0.0f) + (has_yp || ref ? 1.0f : 0.0f) + (has_zm ? 1.0f : 0.0f) +
+                    (has_zp ? 1.0f : 0.0f);
+  struct V { float v[VEC]; };
+  auto ld = [&](const float* a, bool on) {
+    V o;
+    if (VEC == 4) {
+      const float4 f = on ? *reinterpret_cast<const float4*>(a) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      o.v[0] = f.x; o.v[VEC > 1 ? 1 : 0] = f.y; o.v[VEC > 2 ? 2 : 0] = f.z; o.v[VEC > 3 ? 3 : 0] = f.w;
+    } else {
+      o.v[0] = on ? *a : 0.0f;
+    }
+    return o;
+  };
+  const float* xo = x + oth + i;
+  const V cm = ld(xo, true), ym = ld(has_ym ? xo - hx : xo, has_ym), yp = ld(has_yp ? xo + hx : xo, has_yp);
+  const V zm = ld(has_zm ? xo - sz : xo, has_zm), zp = ld(has_zp ? xo + sz : xo, has_zp);
+  const float ex = has_e ? (p == 0 ? xo[-1] : xo[VEC]) : 0.0f;
+  const V xc = ld(x + own + i, true), bv = ld(b + own + i, true);
+  V sv = {};
+  if (TAKE) sv = ld(sum + own + i, true);
+  V out;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) {
+    const float xm = p == 0 ? (j == 0 ? ex : cm.v[j - (j > 0)]) : cm.v[j];
+    const float xp = p == 0 ? cm.v[j] : (j == VEC - 1 ? ex : cm.v[j + (j < VEC - 1)]);
+    const bool edge = !has_e && (p == 0 ? j == 0 : j == VEC - 1);
+    const float diag = dyz + (edge ? 1.0f : 2.0f);
+    const float sumN = ((((xm + xp) + ym.v[j]) + yp.v[j]) + zm.v[j]) + zp.v[j];
+    out.v[j] = bv.v[j] - (sumN - diag * xc.v[j]) * inv_h2;
+    if (TAKE) sv.v[j] = sv.v[j] + xc.v[j];
+  }
+  auto put = [&](float* a, const V& v) {
+    if (VEC == 4)
+      *reinterpret_cast<float4*>(a) = make_float4(v.v[0], v.v[VEC > 1 ? 1 : 0], v.v[VEC > 2 ? 2 : 0], v.v[VEC > 3 ? 3 : 0]);
+    else
+      *a = v.v[0];
+  };
+  put(r + own + i, out);
+  if (TAKE) put(sum + own + i, sv);
+}
+
 // Exact coarsest-grid solve e = M b with the dense symmetric inverse M
 // (n <= 4096 cells).  CTA c forms rows 32c..32c+31 of e: b is gathered into
 // shared memory in natural order, lane l of warp w sums M[i][32c + l] b[i]
@@ -642,7 +795,8 @@ __global__ void k_fill_zero(T* __restrict__ a, size_t n, const unsigned int* __r
 // reads the other colour's finished values, exactly like the reference's
 // single-workgroup solve.
 // A thread's at most kCoarseCells cells of either colour keep their addresses,
-// diagonals and right-hand sides in registers: 6552 cells, 6 sweeps, in 15 us
+// diagonals and right-hand sides in registers.  flip: black first (the
+// transposed sweeps).  6552 cells, 6 sweeps, in 15 us
 // where two CTAs that formed them from the index on every update took 31.
 constexpr int kCoarseThreads = 1024, kCoarseCells = 4;
 constexpr size_t kCoarseSmem = 220 * 1024;  // dynamic shared memory, at most
@@ -657,7 +811,7 @@ inline bool coarse_fits(const Grid& d, int cs) {
 }
 template <class T, int CS>
 __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(kCoarseThreads)
-    k_coarse_sweeps(Grid d, float h2, int ref, int sweeps, T* __restrict__ e, const T* __restrict__ b,
+    k_coarse_sweeps(Grid d, float h2, int ref, int sweeps, int flip, T* __restrict__ e, const T* __restrict__ b,
                     const unsigned int* __restrict__ skip) {
   cg::cluster_group cl = cg::this_cluster();
   extern __shared__ float csm[];  // [2][pzm + 2][ny + 2][hx + 2]
@@ -708,7 +862,8 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(kCoarseThreads)
   const int nsw = skipping ? 0 : sweeps;
   for (int s = 0; s < nsw; ++s) {
 #pragma unroll
-    for (int color = 0; color < 2; ++color) {
+    for (int cc = 0; cc < 2; ++cc) {
+      const int color = cc ^ flip;
       float* own = csm + color * ehalf;
       const float* oth = csm + (1 - color) * ehalf;
 #pragma unroll
@@ -718,7 +873,7 @@ __global__ void __cluster_dims__(CS, 1, 1) __launch_bounds__(kCoarseThreads)
           const int p = par[m] ^ color;
           const float* o = oth + at[m];
           const float sumN = ((((o[p - 1] + o[p]) + o[-kw]) + o[kw]) + o[-pl]) + o[pl];
-          const float v = as_stored<T>((sumN - h2 * bv[m][color]) / (p ? dg[m][1] : dg[m][0]));
+          const float v = as_stored<T>((sumN - h2 * (color ? bv[m][1] : bv[m][0])) / (p ? dg[m][1] : dg[m][0]));
           own[at[m]] = v;
           if (CS > 1) {
             if (at[m] < 2 * pl && dn) dn[color * ehalf + at[m]] = v;
@@ -1242,48 +1397,63 @@ template <int S> static bool leg_narrow(const DevState& s, const Grid& d) {
   return (int)(g.x * g.y * g.z) <= s.num_sms;
 }
 template <class T, class TC, class L>
-static void leg_down_l(const DevState& s, int l, const T* a, const T* b, T* out, TC* bc, const unsigned int* skip,
-                       cudaStream_t st) {
+static void leg_down_l(const DevState& s, int l, const T* a, const T* b, T* out, TC* bc, T* res,
+                       const unsigned int* skip, cudaStream_t st) {
   const MgLevel& V = s.lv[l];
   auto run = [&](auto* k) {
     launch_pdl(k, leg_grid<L>(V.d), dim3(L::NT), 0, st, V.d, s.lv[l + 1].d, V.h2, 1.0f / V.h2, s.ref, a, b, out, bc,
-               skip);
+               res, skip);
   };
-  if (!a) run(k_leg_down<T, TC, L, true>);
-  else if constexpr (sizeof(T) == 4 && sizeof(TC) == 4) run(k_leg_down<T, TC, L, false>);
+  if constexpr (sizeof(T) == 4 && sizeof(TC) == 4) {
+    if (res) run(k_leg_down<T, TC, L, true, true>);
+    else if (a) run(k_leg_down<T, TC, L, false, false>);
+    else run(k_leg_down<T, TC, L, true, false>);
+  } else {
+    run(k_leg_down<T, TC, L, true, false>);
+  }
 }
 template <class T, class TC, class L>
-static void leg_up_l(const DevState& s, int l, const T* a, const T* b, const TC* ec, T* out, const unsigned int* skip,
-                     cudaStream_t st) {
+static void leg_up_l(const DevState& s, int l, const T* a, const T* b, const TC* ec, T* out, bool tr,
+                     const unsigned int* skip, cudaStream_t st) {
   const MgLevel& V = s.lv[l];
-  launch_pdl(k_leg_up<T, TC, L>, leg_grid<L>(V.d), dim3(L::NT), 0, st, V.d, s.lv[l + 1].d, V.h2, s.ref, a, b, ec, out,
-             skip);
+  auto run = [&](auto* k) {
+    launch_pdl(k, leg_grid<L>(V.d), dim3(L::NT), 0, st, V.d, s.lv[l + 1].d, V.h2, s.ref, a, b, ec, out, skip);
+  };
+  if constexpr (sizeof(T) == 4 && sizeof(TC) == 4) {
+    if (tr) {
+      run(k_leg_up<T, TC, L, true>);
+      return;
+    }
+  }
+  run(k_leg_up<T, TC, L, false>);
 }
 // Level l's pre-smoothing (from zero: a null; else FP32 with its first red
 // half-sweep just done, in a) and restriction, and its prolongation and
-// post-smoothing; 1 or 2 sweeps.
+// post-smoothing; 1 or 2 sweeps.  The transposed cycle's (FP32): with res,
+// the smoothing from zero and the black residuals; with tr, the injection and
+// the smoothing.
 template <class T, class TC>
 static void leg_down(const DevState& s, int l, const T* a, const T* b, T* out, TC* bc, int sweeps,
-                     const unsigned int* skip, cudaStream_t st) {
+                     const unsigned int* skip, cudaStream_t st, T* res = nullptr) {
   const Grid& d = s.lv[l].d;
   if (sweeps == 1) {
-    if (leg_narrow<1>(s, d)) leg_down_l<T, TC, LegTile<8, 1>>(s, l, a, b, out, bc, skip, st);
-    else leg_down_l<T, TC, LegTile<16, 1>>(s, l, a, b, out, bc, skip, st);
+    if (leg_narrow<1>(s, d)) leg_down_l<T, TC, LegTile<8, 1>>(s, l, a, b, out, bc, res, skip, st);
+    else leg_down_l<T, TC, LegTile<16, 1>>(s, l, a, b, out, bc, res, skip, st);
   } else {
-    if (leg_narrow<2>(s, d)) leg_down_l<T, TC, LegTile<8, 2>>(s, l, a, b, out, bc, skip, st);
-    else leg_down_l<T, TC, LegTile<16, 2>>(s, l, a, b, out, bc, skip, st);
+    if (leg_narrow<2>(s, d)) leg_down_l<T, TC, LegTile<8, 2>>(s, l, a, b, out, bc, res, skip, st);
+    else leg_down_l<T, TC, LegTile<16, 2>>(s, l, a, b, out, bc, res, skip, st);
   }
 }
 template <class T, class TC>
 static void leg_up(const DevState& s, int l, const T* a, const T* b, const TC* ec, T* out, int sweeps,
-                   const unsigned int* skip, cudaStream_t st) {
+                   const unsigned int* skip, cudaStream_t st, bool tr = false) {
   const Grid& d = s.lv[l].d;
   if (sweeps == 1) {
-    if (leg_narrow<1>(s, d)) leg_up_l<T, TC, LegTile<8, 1>>(s, l, a, b, ec, out, skip, st);
-    else leg_up_l<T, TC, LegTile<16, 1>>(s, l, a, b, ec, out, skip, st);
+    if (leg_narrow<1>(s, d)) leg_up_l<T, TC, LegTile<8, 1>>(s, l, a, b, ec, out, tr, skip, st);
+    else leg_up_l<T, TC, LegTile<16, 1>>(s, l, a, b, ec, out, tr, skip, st);
   } else {
-    if (leg_narrow<2>(s, d)) leg_up_l<T, TC, LegTile<8, 2>>(s, l, a, b, ec, out, skip, st);
-    else leg_up_l<T, TC, LegTile<16, 2>>(s, l, a, b, ec, out, skip, st);
+    if (leg_narrow<2>(s, d)) leg_up_l<T, TC, LegTile<8, 2>>(s, l, a, b, ec, out, tr, skip, st);
+    else leg_up_l<T, TC, LegTile<16, 2>>(s, l, a, b, ec, out, tr, skip, st);
   }
 }
 static bool leg_sweeps_ok(int pre, int post) { return (pre == 1 || pre == 2) && (post == 1 || post == 2); }
@@ -1362,9 +1532,10 @@ static void half_sweep(const DevState& s, int l, int c, bool zoth, T* a, const T
 // there are no sweeps); ec: coarse correction to add first.
 // red_done: the first red half-sweep from zero was formed by the restriction
 // into this level (restrict_level's ered)
+// flip: black before red (the transposed sweeps)
 template <class T, class TC = T>
 static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, bool zero_first, const TC* ec,
-                   const unsigned int* skip, cudaStream_t st, bool red_done = false) {
+                   const unsigned int* skip, cudaStream_t st, bool red_done = false, int flip = 0) {
   const MgLevel& L = s.lv[l];
   if (zero_first && sweeps == 0) launch_pdl(k_fill_zero<T>, dim3(s.num_sms * 2), dim3(256), 0, st, a, L.d.n(), skip);
   if (ec) {
@@ -1388,12 +1559,13 @@ static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, bool 
   for (int k = 0; k < sweeps; ++k)
     for (int c = 0; c < 2; ++c) {
       if (red_done && k == 0 && c == 0) continue;
-      half_sweep<T>(s, l, c, zero_first && k == 0 && c == 0, a, b, skip, st);
+      half_sweep<T>(s, l, c ^ flip, zero_first && k == 0 && c == 0, a, b, skip, st);
     }
 }
 
 template <class T>
-static void coarse_solve(const DevState& s, int l, T* e, const T* b, const unsigned int* skip, cudaStream_t st) {
+static void coarse_solve(const DevState& s, int l, T* e, const T* b, const unsigned int* skip, cudaStream_t st,
+                         int flip = 0) {
   const MgLevel& L = s.lv[l];
   if (s.coarse_sweeps < 0) {  // exact: e = M b with the precomputed inverse
     if (s.cn <= 32 * kDenseChain)
@@ -1406,11 +1578,11 @@ static void coarse_solve(const DevState& s, int l, T* e, const T* b, const unsig
   // one CTA where its threads hold the grid, else a cluster of eight
   auto run = [&](auto* k, int cs) {
     launch_pdl(k, dim3(cs), dim3(kCoarseThreads), coarse_words(L.d, cs) * sizeof(float), st, L.d, L.h2, s.ref,
-               s.coarse_sweeps, e, b, skip);
+               s.coarse_sweeps, flip, e, b, skip);
   };
   if (coarse_fits(L.d, 1)) run(k_coarse_sweeps<T, 1>, 1);
   else if (coarse_fits(L.d, 8)) run(k_coarse_sweeps<T, 8>, 8);
-  else smooth<T, T>(s, l, e, b, s.coarse_sweeps, true, nullptr, skip, st);
+  else smooth<T, T>(s, l, e, b, s.coarse_sweeps, true, nullptr, skip, st, false, flip);
 }
 
 // One V-cycle on (x0, b0); per-level arrays E[l], B[l] for l >= 1.
@@ -1458,6 +1630,91 @@ static void vcycle(const DevState& s, T* x0, const T* b0, T* const* E, T* const*
   }
   if (leg0) leg_up<T, T>(s, 0, s.lv[0].e2, b0, X[1], x0, s.post0, skip, st);
   else smooth<T, T>(s, 0, x0, b0, s.post0, false, X[1], skip, st);
+}
+
+// The transposed V-cycle.  A cycle of vcycle() is p + N (b - A p) with N
+// linear, so its transpose takes the adjoint ap of p and arhs of b to
+// arhs + N^T ap and ap - A N^T ap (A is symmetric).  N^T is itself a V-cycle
+// from zero: the post-smoothing's sweeps with the colours exchanged (a
+// half-sweep is its own transpose, the order turns round), the transposed
+// prolongation for a restriction, the transposed coarsest solve, the
+// transposed average for a prolongation, and the pre-smoothing's sweeps with
+// the colours exchanged.  So it runs on the forward cycle's kernels and level
+// arrays, one launch per leg on the small levels, and one residual pass ends
+// it (96x128x96, a backward step of four cycles: 969 -> 759 us against
+// half-sweeps transposed one by one, which update the right-hand side's
+// adjoint in every launch).  x0, t0: two arrays of the finest grid's size, R[l] one of every other
+// level's (residuals).
+static void transposed_cycle(const DevState& s, float* ap, float* arhs, float* x0, float* t0, float* const* R,
+                             cudaStream_t st) {
+  const int L = s.nlev;
+  float* X[kMaxLevels];
+  const float* B[kMaxLevels];
+  for (int l = 0; l < L; ++l) {
+    X[l] = l ? s.lv[l].e : x0;
+    B[l] = l ? s.lv[l].b : ap;
+  }
+  if (L == 1) {
+    smooth<float, float>(s, 0, x0, ap, s.pre + s.post, true, nullptr, nullptr, st, false, 1);
+  } else {
+    for (int l = 0; l < L - 1; ++l) {
+      const Grid f = s.lv[l].d, c = s.lv[l + 1].d;
+      const int sweeps = l ? s.post : s.post0;
+      float* r = l ? R[l] : t0;
+      const float* from = r;
+      if (leg_ok(s, l)) {
+        leg_down<float, float>(s, l, nullptr, B[l], X[l], nullptr, sweeps, nullptr, st, r);
+      } else {
+        smooth<float, float>(s, l, X[l], B[l], sweeps, true, nullptr, nullptr, st, false, 1);
+        const float inv_h2 = 1.0f / s.lv[l].h2;
+        if (sweeps == 0) {
+          from = B[l];  // x = 0: the residual is the right-hand side
+        } else if (f.nx % 8 == 0) {
+          const dim3 bq = quad_block(f);
+          launch_pdl(k_residual_t<false, 4>, quad_grid(f, bq), bq, 0, st, f, inv_h2, s.ref, (const float*)X[l], B[l],
+                     r, (float*)nullptr);
+        } else {
+          launch_pdl(k_residual_t<false, 1>, g_half(f), b_cells(), 0, st, f, inv_h2, s.ref, (const float*)X[l], B[l],
+                     r, (float*)nullptr);
+        }
+      }
+      const dim3 bp = pair_block(c);
+      if (sweeps > 0) launch_pdl(k_prolong_t2<true>, pair_grid(c, bp), bp, 0, st, f, c, s.ref, from, s.lv[l + 1].b);
+      else launch_pdl(k_prolong_t2<false>, pair_grid(c, bp), bp, 0, st, f, c, s.ref, from, s.lv[l + 1].b);
+    }
+    coarse_solve<float>(s, L - 1, X[L - 1], B[L - 1], nullptr, st, 1);
+    for (int l = L - 2; l >= 0; --l) {
+      const Grid f = s.lv[l].d, c = s.lv[l + 1].d;
+      const int sweeps = l ? s.pre : s.pre0;
+      if (leg_ok(s, l)) {
+        float* out = l ? s.lv[l].e2 : t0;
+        leg_up<float, float>(s, l, X[l], B[l], X[l + 1], out, sweeps, nullptr, st, true);
+        X[l] = out;
+        continue;
+      }
+      const dim3 bp = pair_block(c);
+      const dim3 gp((c.nx / 2 + bp.x - 1) / bp.x, (f.ny + bp.y - 1) / bp.y, f.nz);
+      if (sweeps > 0) launch_pdl(k_inject_t2<true>, gp, bp, 0, st, f, c, X[l], (const float*)X[l + 1]);
+      else launch_pdl(k_inject_t2<false>, gp, bp, 0, st, f, c, X[l], (const float*)X[l + 1]);
+      smooth<float, float>(s, l, X[l], B[l], sweeps, false, nullptr, nullptr, st, false, 1);
+    }
+  }
+  const Grid d = s.g;
+  if (d.nx % 8 == 0) {
+    const dim3 bq = quad_block(d);
+    dim3 gq = quad_grid(d, bq);
+    gq.z = 2 * d.nz;
+    launch_pdl(k_residual_t<true, 4>, gq, bq, 0, st, d, 1.0f, s.ref, (const float*)X[0], (const float*)ap, ap, arhs);
+  } else {
+    dim3 gh = g_half(d);
+    gh.z = 2 * d.nz;
+    launch_pdl(k_residual_t<true, 1>, gh, b_cells(), 0, st, d, 1.0f, s.ref, (const float*)X[0], (const float*)ap, ap,
+               arhs);
+  }
+}
+void launch_transposed_cycles(const DevState& s, float* ap, float* arhs, float* x0, float* t0, float* const* R,
+                              cudaStream_t st) {
+  for (int c = 0; c < s.cycles; ++c) transposed_cycle(s, ap, arhs, x0, t0, R, st);
 }
 
 // ---- the mixed-precision correction solve --------------------------------------------------
