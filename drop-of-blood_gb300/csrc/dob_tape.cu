@@ -357,9 +357,9 @@ void backward_step(dob_ctx* ctx, int j) {
   launch_adj_pressure_solve(t, a, st);
   launch_adj_mac_rhs(t, a, st);
   cudaMemsetAsync(a.arhs, 0, N * 4, st);
-  // Casson viscosity, linearised at (u after advection, dye_j)
+  // Casson viscosity, linearised at (u after advection, dye_j); the arrays it
+  // adds to are zero: the step before (or zero_adj) left them so
   swap3(a.au, a.av, a.aw, a.au2, a.av2, a.aw2);
-  for (float* p : {a.au, a.av, a.aw}) cudaMemsetAsync(p, 0, N * 4, st);
   t.u = A->Tua[j]; t.v = A->Tva[j]; t.w = A->Twa[j]; t.conc = A->Tc[j];
   launch_adj_casson(t, a, st);
   // advection, linearised at (u_j, cen_j)
