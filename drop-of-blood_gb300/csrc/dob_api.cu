@@ -170,6 +170,18 @@ static dob_status upload_params(dob_ctx* ctx, uint32_t spawn) {
   return DOB_OK;
 }
 
+// The uniform block of the next step for its wave substep (same ring).
+static dob_status upload_next(dob_ctx* ctx, const float* U) {
+  const int k = ctx->param_slot;
+  ctx->param_slot = (k + 1) % kParamRing;
+  CK(cudaEventSynchronize(ctx->param_ev[k]));
+  memcpy(ctx->host_params[k].U, U, sizeof(ctx->host_params[k].U));
+  CK(cudaMemcpyAsync(ctx->next_params->U, ctx->host_params[k].U, sizeof(ctx->host_params[k].U),
+                     cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaEventRecord(ctx->param_ev[k], ctx->stream));
+  return DOB_OK;
+}
+
 static void swap_vel(DevState& s) {
   std::swap(s.u, s.u2);
   std::swap(s.v, s.v2);
@@ -212,8 +224,13 @@ static const int kStepOrder[] = {
 // projected centre velocity and the dye, beside the dye predictor; it joins
 // before the resolve in reference mode, which reads the splats, and at the
 // step's end in the closed box.
+// wave_done / wave_next (with side): the wave substep of this step has run
+// already, and the next step's runs here: it reads the projected v faces and
+// the next step's uniform block, and nothing after the projection reads or
+// writes the wave field, so its four small kernels run beside the parcels
+// and the dye.
 static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float* stage_ms, bool stats_div,
-                              cudaStream_t side = nullptr) {
+                              cudaStream_t side = nullptr, bool wave_done = false, bool wave_next = false) {
   const int n = (int)(sizeof(kStepOrder) / sizeof(kStepOrder[0]));
   auto order = [&](int ev, cudaStream_t first, cudaStream_t then) {  // `then` goes on after the work on `first`
     cudaEventRecord(ctx->side_ev[ev], first);
@@ -227,7 +244,7 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
   }
   // the wave substep comes first and the advection reads its result
   // (BloodDropEngine.ts:1886-1912)
-  if (s.flags & DOB_PHYS_WAVE) launch_wave_step(s, st);
+  if ((s.flags & DOB_PHYS_WAVE) && !wave_done) launch_wave_step(s, st);
   if (side) {
     order(1, st, side);
     launch_parcel_emit(s, side);
@@ -266,6 +283,13 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
       launch_project_center_ref(s, st);
       swap_vel(s);
       centre_fused = true;
+      if (wave_next) {
+        order(1, st, ctx->wave_stream);
+        DevState next = s;
+        next.params = ctx->next_params;
+        launch_wave_step(next, ctx->wave_stream);
+        cudaEventRecord(ctx->side_ev[4], ctx->wave_stream);
+      }
     } else if (!s.ref && stage == DOB_STAGE_MAC_RHS) {
       // with statistics the mean removal also forms ||rhs||^2
       if (stats_div) cudaMemsetAsync(s.red + RED_RHS_NORM2, 0, sizeof(double), st);
@@ -309,6 +333,7 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
     }
   }
   if (side && !s.ref) cudaStreamWaitEvent(st, ctx->side_ev[3], 0);
+  if (wave_next) cudaStreamWaitEvent(st, ctx->side_ev[4], 0);
 }
 
 // Graphs are cached per (statistics on/off, dye and velocity buffers at the
@@ -322,12 +347,14 @@ static void pingpong_set(DevState& s, void* const* in) {
   s.conc = in[6]; s.conc2 = in[7];
 }
 
-static dob_status get_graph(dob_ctx* ctx, bool stats, bool injected, dob_ctx::StepGraph** out) {
+static dob_status get_graph(dob_ctx* ctx, bool stats, bool injected, bool wave_done, bool wave_next,
+                            dob_ctx::StepGraph** out) {
   const int nslots = (int)(sizeof(ctx->graphs) / sizeof(ctx->graphs[0]));
   int slot = -1;
   for (int k = 0; k < nslots; ++k) {
     dob_ctx::StepGraph& G = ctx->graphs[k];
-    if (G.ex && G.stats == stats && G.injected == injected && G.conc == ctx->s.conc && G.u == ctx->s.u) {
+    if (G.ex && G.stats == stats && G.injected == injected && G.wave_done == wave_done && G.wave_next == wave_next &&
+        G.conc == ctx->s.conc && G.u == ctx->s.u) {
       *out = &G;
       return DOB_OK;
     }
@@ -343,7 +370,7 @@ static dob_status get_graph(dob_ctx* ctx, bool stats, bool injected, dob_ctx::St
   if (injected) s.cycles = ctx->cfg.mg_cycles_injected;
   cudaGraph_t g = nullptr;
   CK(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  enqueue_step_body(ctx, s, ctx->stream, nullptr, stats, ctx->side_stream);
+  enqueue_step_body(ctx, s, ctx->stream, nullptr, stats, ctx->side_stream, wave_done, wave_next);
   cudaError_t e = cudaStreamEndCapture(ctx->stream, &g);
   if (e != cudaSuccess) return fail(ctx, DOB_ECUDA, "cudaStreamEndCapture", cudaGetErrorString(e));
   size_t nn = 0;
@@ -355,7 +382,7 @@ static dob_status get_graph(dob_ctx* ctx, bool stats, bool injected, dob_ctx::St
     cudaGraphNodeType t;
     if (cudaGraphNodeGetType(nodes[k], &t) == cudaSuccess && t == cudaGraphNodeTypeKernel) ++kernels;
   }
-  if (!stats) ctx->kernels_per_step = kernels;
+  if (!stats && wave_done == wave_next) ctx->kernels_per_step = kernels;
   cudaGraphExec_t ex = nullptr;
   e = cudaGraphInstantiate(&ex, g, 0);
   cudaGraphDestroy(g);
@@ -364,6 +391,8 @@ static dob_status get_graph(dob_ctx* ctx, bool stats, bool injected, dob_ctx::St
   G.ex = ex;
   G.stats = stats;
   G.injected = injected;
+  G.wave_done = wave_done;
+  G.wave_next = wave_next;
   G.conc = ctx->s.conc;
   G.u = ctx->s.u;
   pingpong_get(s, G.after);
@@ -379,7 +408,10 @@ static void drop_graphs(dob_ctx* ctx) {
   ctx->graph_next = 0;
 }
 
-static dob_status one_step(dob_ctx* ctx, uint32_t flags, float* stage_ms) {
+// wave_done (in and out): whether the wave substep of this step (then: of the
+// next) has run.  next: the uniform block of a step that follows in the same
+// call, or null; its wave substep may then run beside this step.
+static dob_status one_step(dob_ctx* ctx, uint32_t flags, float* stage_ms, bool* wave_done, const float* next) {
   const uint32_t spawn = spawn_count(ctx);
   if (ctx->cfg.bc_mode == DOB_BC_REFERENCE) {  // BloodDropEngine.ts:1832-1840
     const uint64_t hw = (uint64_t)ctx->high_water + spawn;
@@ -400,10 +432,13 @@ static dob_status one_step(dob_ctx* ctx, uint32_t flags, float* stage_ms) {
     enqueue_step_body(ctx, ctx->s, ctx->stream, stage_ms, stats);
     ctx->s.cycles = cycles;
   } else {
+    const bool wave_next = next && (ctx->s.flags & DOB_PHYS_WAVE);
+    if (wave_next && (st = upload_next(ctx, next)) != DOB_OK) return st;
     dob_ctx::StepGraph* G = nullptr;
-    st = get_graph(ctx, stats, injected, &G);
+    st = get_graph(ctx, stats, injected, *wave_done, wave_next, &G);
     if (st != DOB_OK) return st;
     CK(cudaGraphLaunch(G->ex, ctx->stream));
+    *wave_done = wave_next;
     pingpong_set(ctx->s, G->after);  // the buffers the captured step wrote last
   }
   CK(cudaGetLastError());
@@ -532,6 +567,7 @@ dob_status dob_create(const dob_config* cfg, dob_ctx** out) {
   int prio_low = 0, prio_high = 0;
   CK(cudaDeviceGetStreamPriorityRange(&prio_low, &prio_high));
   CK(cudaStreamCreateWithPriority(&ctx->side_stream, cudaStreamNonBlocking, prio_high));
+  CK(cudaStreamCreateWithPriority(&ctx->wave_stream, cudaStreamNonBlocking, prio_high));
   for (cudaEvent_t& ev : ctx->side_ev) CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
   CK(mg_prepare());
   s.aux = ctx->aux_stream;
@@ -567,6 +603,7 @@ dob_status dob_create(const dob_config* cfg, dob_ctx** out) {
   if (s.flags & DOB_PHYS_WAVE) {
     A((void**)&s.wspec, (size_t)kWaveN * kWaveN * 8);
     A((void**)&s.wfilm, (size_t)kWaveN * kWaveN * 4);
+    A((void**)&ctx->next_params, sizeof(StepParams));
   }
   A((void**)&s.parcels, (size_t)s.cap * 32);
   if (s.ref && light_dims_ok(s.g)) {
@@ -679,6 +716,7 @@ void dob_destroy(dob_ctx* ctx) {
   if (ctx->aux_stream) cudaStreamDestroy(ctx->aux_stream);
   if (ctx->aux_stream2) cudaStreamDestroy(ctx->aux_stream2);
   if (ctx->side_stream) cudaStreamDestroy(ctx->side_stream);
+  if (ctx->wave_stream) cudaStreamDestroy(ctx->wave_stream);
   for (cudaEvent_t ev : ctx->side_ev)
     if (ev) cudaEventDestroy(ev);
   delete ctx;
@@ -944,15 +982,17 @@ dob_status dob_get_field(dob_ctx* ctx, int field, void* host, size_t bytes) {
 
 // ---- stepping ----------------------------------------------------------------------------
 // `light`: end with the lighting passes (DOB_PHYS_LIGHTING), which read the
-// last step's parameters.
-static dob_status step_impl(dob_ctx* ctx, int nsteps, uint32_t flags, dob_step_stats* stats, bool light) {
+// last step's parameters.  wave_done, next: as one_step's, across calls of
+// one dob_step_uniforms (next: the block after these steps, or null).
+static dob_status step_impl(dob_ctx* ctx, int nsteps, uint32_t flags, dob_step_stats* stats, bool light,
+                            bool* wave_done, const float* next) {
   if (!ctx || nsteps < 0) return DOB_EINVAL;
   if (ctx->cfg.bc_mode == DOB_BC_REFERENCE && !isfinite(ctx->U[38]))
     return fail(ctx, DOB_EINVAL, "dob_step", "non-finite dt");
   float stage_ms[DOB_STAGE_COUNT] = {0};
   const bool timing = (flags & DOB_STEP_TIMING) != 0;
   for (int k = 0; k < nsteps; ++k) {
-    dob_status st = one_step(ctx, flags, timing ? stage_ms : nullptr);
+    dob_status st = one_step(ctx, flags, timing ? stage_ms : nullptr, wave_done, k + 1 < nsteps ? ctx->U : next);
     if (st != DOB_OK) return st;
   }
   if (light && nsteps > 0 && ctx->s.light && (ctx->s.flags & DOB_PHYS_LIGHTING)) {
@@ -975,7 +1015,8 @@ static dob_status step_impl(dob_ctx* ctx, int nsteps, uint32_t flags, dob_step_s
 }
 
 dob_status dob_step(dob_ctx* ctx, int nsteps, uint32_t flags, dob_step_stats* stats) {
-  return step_impl(ctx, nsteps, flags, stats, true);
+  bool wave_done = false;
+  return step_impl(ctx, nsteps, flags, stats, true, &wave_done, nullptr);
 }
 
 dob_status dob_step_async(dob_ctx* ctx, int slot) {
@@ -989,7 +1030,8 @@ dob_status dob_step_async(dob_ctx* ctx, int slot) {
     a.redu = reinterpret_cast<unsigned int*>(a.red + RED_COUNT);
     CK(cudaEventCreateWithFlags(&a.done, cudaEventDisableTiming));
   }
-  dob_status st = one_step(ctx, DOB_STEP_STATS, nullptr);
+  bool wave_done = false;
+  dob_status st = one_step(ctx, DOB_STEP_STATS, nullptr, &wave_done, nullptr);
   if (st != DOB_OK) return st;
   DevState& s = ctx->s;
   if (ctx->stats_mask & DOB_STATS_PARCELS) launch_count_alive(s, s.redu + REDU_ALIVE, ctx->stream);
@@ -1025,10 +1067,19 @@ dob_status dob_step_result(dob_ctx* ctx, int slot, dob_step_stats* stats) {
 
 dob_status dob_step_uniforms(dob_ctx* ctx, const float* blocks, int nsteps, uint32_t flags, dob_step_stats* stats) {
   if (!ctx || (!blocks && nsteps) || nsteps < 0) return DOB_EINVAL;
+  auto finite = [](const float* u) {
+    for (int k = 0; k < 128; ++k)
+      if (!isfinite(u[k])) return false;
+    return true;
+  };
+  bool wave_done = false;
   for (int k = 0; k < nsteps; ++k) {
     dob_status st = dob_set_uniforms(ctx, blocks + (size_t)k * 128);
     if (st != DOB_OK) return st;
-    st = step_impl(ctx, 1, flags, k == nsteps - 1 ? stats : nullptr, k == nsteps - 1);
+    // a block that its own step will refuse is not used before it
+    const float* next = k + 1 < nsteps ? blocks + (size_t)(k + 1) * 128 : nullptr;
+    if (next && !finite(next)) next = nullptr;
+    st = step_impl(ctx, 1, flags, k == nsteps - 1 ? stats : nullptr, k == nsteps - 1, &wave_done, next);
     if (st != DOB_OK) return st;
   }
   return DOB_OK;
@@ -1123,7 +1174,7 @@ dob_status dob_launches_per_step(dob_ctx* ctx, int* n) {
   if (!ctx->kernels_per_step) {
     // capture the plain step graph once (no launch) to count its kernel nodes
     dob_ctx::StepGraph* G = nullptr;
-    dob_status st = get_graph(ctx, false, false, &G);
+    dob_status st = get_graph(ctx, false, false, false, false, &G);
     if (st != DOB_OK) return st;
   }
   *n = ctx->kernels_per_step;
@@ -1147,8 +1198,10 @@ dob_status dob_time_steps(dob_ctx* ctx, int nsteps, uint32_t flags, float* ms) {
   if (!ctx || !ms || nsteps < 0) return DOB_EINVAL;
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaEventRecord(ctx->ev0, ctx->stream));
+  bool wave_done = false;
   for (int k = 0; k < nsteps; ++k) {
-    dob_status st = one_step(ctx, flags & ~(uint32_t)DOB_STEP_TIMING, nullptr);
+    dob_status st = one_step(ctx, flags & ~(uint32_t)DOB_STEP_TIMING, nullptr, &wave_done,
+                             k + 1 < nsteps ? ctx->U : nullptr);
     if (st != DOB_OK) return st;
   }
   CK(cudaEventRecord(ctx->ev1, ctx->stream));

@@ -40,10 +40,13 @@ struct dob_ctx {
   cudaStream_t stream = nullptr;
   cudaStream_t aux_stream = nullptr;   // body capture of conditional graph nodes
   cudaStream_t aux_stream2 = nullptr;  // the same, one nesting level up
-  // second branch of a captured step (enqueue_step_body) and the events that
-  // fork and join it; used in stream capture only
-  cudaStream_t side_stream = nullptr;
-  cudaEvent_t side_ev[4] = {};
+  // further branches of a captured step (enqueue_step_body) and the events
+  // that fork and join them; used in stream capture only
+  cudaStream_t side_stream = nullptr, wave_stream = nullptr;
+  cudaEvent_t side_ev[5] = {};
+  // parameters of the step after the current one, as far as its wave substep
+  // reads them (the uniform block), when that runs beside this step's tail
+  dob::StepParams* next_params = nullptr;
   std::string err;
   float U[128];
   dob::StepParams* host_params = nullptr;  // pinned ring
@@ -60,9 +63,12 @@ struct dob_ctx {
     cudaGraphExec_t ex = nullptr;
     bool stats = false;
     bool injected = false;  // captured with mg_cycles_injected V-cycles
+    // the wave substep has run in the step before, this step runs the next
+    // step's (DOB_PHYS_WAVE, steps of one call)
+    bool wave_done = false, wave_next = false;
     void *conc = nullptr, *u = nullptr;
     void* after[8] = {};  // u, v, w, u2, v2, w2, conc, conc2
-  } graphs[12];
+  } graphs[24];
   int graph_next = 0;  // round-robin replacement when all slots are taken
   // steps left that run cfg.mg_cycles_injected V-cycles (when set and the
   // pressure is FP32): an injection sets kInjectedSteps
