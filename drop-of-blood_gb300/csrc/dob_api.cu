@@ -18,8 +18,11 @@
 #include <math.h>
 #include <stdio.h>
 #include <string.h>
+#include <sys/mman.h>
+#include <unistd.h>
 
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "dob_kernels.cuh"
@@ -478,6 +481,30 @@ static dob_status finish_stats(dob_ctx* ctx, dob_step_stats* stats, int steps) {
   return DOB_OK;
 }
 
+// ---- field readback ----
+// What a field that is not FP32 in natural order holds on the device.
+enum FieldForm { kHalfForm, kSplitForm, kSplitPairForm };
+
+// out = elements [i0, i0 + n) of a field, as FP32 in natural order.  Bound by
+// the copy that follows each piece.  Binary16 was converted on one host thread
+// before: 8.3 ms for 9.4 million values, 1.5 now, page populating included.
+template <int FORM>
+__global__ void __launch_bounds__(256) k_field_to_f32(const void* __restrict__ field, const float* __restrict__ lo,
+                                                      Grid d, size_t i0, size_t n, float* __restrict__ out) {
+  for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n; k += (size_t)gridDim.x * blockDim.x) {
+    const size_t i = i0 + k;
+    if (FORM == kHalfForm) {
+      out[k] = dob_f16_bits_to_f32(((const uint16_t*)field)[i]);
+    } else {
+      const size_t row = i / d.nx;
+      const int x = (int)(i - row * d.nx), z = (int)(row / d.ny), y = (int)(row - (size_t)z * d.ny);
+      const size_t r = rb_index(d, x, y, z);
+      const float v = ((const float*)field)[r];
+      out[k] = FORM == kSplitPairForm ? v + lo[r] : v;
+    }
+  }
+}
+
 extern "C" {
 
 int dob_abi_version(void) { return DOB_ABI_VERSION; }
@@ -583,6 +610,7 @@ dob_status dob_create(const dob_config* cfg, dob_ctx** out) {
   dob_status st = DOB_OK;
   auto A = [&](void** p, size_t b) { if (st == DOB_OK) st = dev_alloc(ctx, p, b); };
   A((void**)&s.params, sizeof(StepParams));
+  A((void**)&ctx->stage, kStageFloats * sizeof(float));
   A(&s.u, N * vsb); A(&s.v, N * vsb); A(&s.w, N * vsb);
   A(&s.u2, N * vsb); A(&s.v2, N * vsb); A(&s.w2, N * vsb);
   A(&s.cen, N * 4 * vsb);
@@ -825,9 +853,47 @@ dob_status dob_set_parcels(dob_ctx* ctx, const float* p, uint32_t n, uint32_t of
   return DOB_OK;
 }
 
+// Back the pages of a host buffer about to be written whole with memory.  A
+// fresh buffer (a new numpy array) has none, and cudaMemcpy then faults them in
+// one by one: 2.6 ms for 38 MB against 0.2 ms of copying.  Populating takes 0.9
+// ms on one thread and 0.6 on four, 151 MB 4.5 and 1.4 (eight: 1.5); buffers
+// below 8 MB mostly come from the allocator's warm pages.  Called before the
+// wait for the stream, so that it runs beside the steps still in flight.  A
+// hint only: nothing is written, and what the call does not take (device,
+// pinned or file memory, an old kernel) is left to the copy.
+static void populate_pages(void* host, size_t bytes) {
+#ifdef MADV_POPULATE_WRITE
+  if (bytes < ((size_t)8 << 20)) return;
+  const uintptr_t page = (uintptr_t)sysconf(_SC_PAGESIZE);
+  const uintptr_t lo = (uintptr_t)host & ~(page - 1), hi = ((uintptr_t)host + bytes + page - 1) & ~(page - 1);
+  const size_t hw = std::thread::hardware_concurrency();
+  size_t parts = bytes >> 24;  // a thread for every 16 MB, up to four
+  if (parts > 4) parts = 4;
+  if (parts > hw) parts = hw;
+  if (parts < 1) parts = 1;
+  const uintptr_t step = ((hi - lo) / parts + page - 1) & ~(page - 1);
+  auto part = [=](size_t k) {
+    const uintptr_t a = lo + k * step, b = k + 1 < parts ? a + step : hi;
+    if (a < b) madvise((void*)a, b - a, MADV_POPULATE_WRITE);
+  };
+  std::thread helpers[3];
+  size_t started = 0;
+  try {
+    for (; started + 1 < parts; ++started) helpers[started] = std::thread(part, started + 1);
+  } catch (...) {  // no thread to be had: the copy faults those pages in
+  }
+  part(0);
+  for (size_t k = 0; k < started; ++k) helpers[k].join();
+#else
+  (void)host;
+  (void)bytes;
+#endif
+}
+
 dob_status dob_get_parcels(dob_ctx* ctx, float* p, uint32_t n, uint32_t off) {
   if (!ctx || (!p && n)) return DOB_EINVAL;
   if ((uint64_t)off + n > ctx->s.cap) return fail(ctx, DOB_EINVAL, "dob_get_parcels", "range exceeds capacity");
+  populate_pages(p, (size_t)n * 32);
   CK(cudaStreamSynchronize(ctx->stream));
   CK(cudaMemcpy(p, ctx->s.parcels + (size_t)off * 8, (size_t)n * 32, cudaMemcpyDeviceToHost));
   return DOB_OK;
@@ -848,12 +914,6 @@ static dob_status dye_bricks_unknown(dob_ctx* ctx) {
 }
 
 // ---- field I/O -----------------------------------------------------------------------
-__global__ void k_add_arrays(const float* __restrict__ a, const float* __restrict__ b, float* __restrict__ out,
-                             size_t n) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-    out[i] = a[i] + b[i];
-}
-
 namespace {
 struct FieldDesc {
   void* dev;
@@ -931,8 +991,8 @@ dob_status dob_set_field(dob_ctx* ctx, int field, const void* host, size_t bytes
 
 dob_status dob_get_field(dob_ctx* ctx, int field, void* host, size_t bytes) {
   if (!ctx || !host) return DOB_EINVAL;
-  CK(cudaStreamSynchronize(ctx->stream));
   if (field == DOB_FIELD_DIVERGENCE) {
+    CK(cudaStreamSynchronize(ctx->stream));
     const size_t N = ctx->s.g.n();
     if (bytes != N * 4) return fail(ctx, DOB_EINVAL, "dob_get_field", "byte count does not match the field");
     float* tmp = nullptr;
@@ -948,35 +1008,24 @@ dob_status dob_get_field(dob_ctx* ctx, int field, void* host, size_t bytes) {
   if (!field_desc(ctx, field, &f)) return fail(ctx, DOB_EINVAL, "dob_get_field", "unknown field");
   if (bytes != f.count * 4) return fail(ctx, DOB_EINVAL, "dob_get_field", "byte count does not match the field");
   const size_t eb = f.kind == 0 ? vs_bytes(ctx->s.prec) : f.kind == 1 ? ds_bytes(ctx->s.prec) : f.kind == 5 ? 2 : 4;
-  if (f.kind == 4) {
-    float* tmp = nullptr;
-    CK(cudaMalloc(&tmp, bytes));
-    cudaError_t e = cudaSuccess;
-    if (field == DOB_FIELD_PRESSURE && ctx->s.plo) {
-      // double-float pressure: read p + plo rounded to FP32
-      float* sum = nullptr;
-      e = cudaMalloc(&sum, bytes);
-      if (e == cudaSuccess) {
-        k_add_arrays<<<ctx->s.num_sms * 4, 256, 0, ctx->stream>>>(ctx->s.p, ctx->s.plo, sum, f.count);
-        launch_split(sum, tmp, ctx->s.g, false, ctx->stream);
-        e = cudaStreamSynchronize(ctx->stream);
-        cudaFree(sum);
-      }
-    } else {
-      launch_split((const float*)f.dev, tmp, ctx->s.g, false, ctx->stream);
-    }
-    if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    if (e == cudaSuccess) e = cudaMemcpy(host, tmp, bytes, cudaMemcpyDeviceToHost);
-    cudaFree(tmp);
-    if (e != cudaSuccess) return fail(ctx, DOB_ECUDA, "dob_get_field", cudaGetErrorString(e));
-  } else if (eb == 4) {
+  populate_pages(host, bytes);
+  CK(cudaStreamSynchronize(ctx->stream));
+  if (f.kind == 2 || f.kind == 3 || (f.kind != 4 && eb == 4)) {
     CK(cudaMemcpy(host, f.dev, bytes, cudaMemcpyDeviceToHost));
-  } else {
-    std::vector<uint16_t> tmp(f.count);
-    CK(cudaMemcpy(tmp.data(), f.dev, f.count * 2, cudaMemcpyDeviceToHost));
-    float* dst = (float*)host;
-    for (size_t i = 0; i < f.count; ++i) dst[i] = dob_f16_bits_to_f32(tmp[i]);
+    return DOB_OK;
   }
+  const float* lo = field == DOB_FIELD_PRESSURE ? ctx->s.plo : nullptr;  // read p + plo, rounded to FP32
+  for (size_t i0 = 0; i0 < f.count; i0 += kStageFloats) {
+    const size_t n = f.count - i0 < kStageFloats ? f.count - i0 : kStageFloats;
+    const int blocks = ctx->s.num_sms * 8;
+    auto convert = f.kind != 4 ? k_field_to_f32<kHalfForm>
+                   : lo        ? k_field_to_f32<kSplitPairForm>
+                               : k_field_to_f32<kSplitForm>;
+    convert<<<blocks, 256, 0, ctx->stream>>>(f.dev, lo, ctx->s.g, i0, n, ctx->stage);
+    CK(cudaGetLastError());
+    CK(cudaMemcpyAsync((float*)host + i0, ctx->stage, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
+  }
+  CK(cudaStreamSynchronize(ctx->stream));
   return DOB_OK;
 }
 

@@ -19,6 +19,9 @@ constexpr int kSnapshots = 8;
 // step's pressure leaves max |div| near 7e-5 after 4 V-cycles at 192 x 256
 // x 192; the third step is back below 2e-6).
 constexpr int kInjectedSteps = 2;
+// Readback of what is not FP32 in natural order goes through a buffer of 8 MB
+// piece by piece: a piece's copy (45 us) is well above its two launches.
+constexpr size_t kStageFloats = (size_t)2 << 20;
 
 struct Snapshot {
   std::vector<void*> bufs;
@@ -93,6 +96,7 @@ struct dob_ctx {
   float4* lut = nullptr;
   __half* image = nullptr;
   size_t image_cap = 0;
+  float* stage = nullptr;  // kStageFloats
   int render_w = 0, render_h = 0;  // the last render's size (dob_bench_kernel 3)
 };
 
