@@ -200,7 +200,7 @@ static void enqueue_stage(dob_ctx* ctx, DevState& s, int stage, cudaStream_t st,
     case DOB_STAGE_ADVECT_MAC: launch_advect_mac(s, st); swap_vel(s); break;
     case DOB_STAGE_MAC_TO_CENTER: launch_mac_to_center(s, st); break;
     case DOB_STAGE_CURL: if (s.curl) launch_curl(s, st); break;
-    case DOB_STAGE_CASSON_FORCES: launch_casson(s, st); swap_vel(s); break;
+    case DOB_STAGE_CASSON_FORCES: launch_casson(s, st, in_step); swap_vel(s); break;
     case DOB_STAGE_MAC_RHS: launch_mac_rhs(s, st); break;
     case DOB_STAGE_PRESSURE_SOLVE: launch_pressure_solve(s, st); break;
     case DOB_STAGE_PROJECT: launch_project(s, st); break;
@@ -241,9 +241,11 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
   };
   if (side) {
     order(0, st, side);
-    launch_dye_flags_clear(s, side);
+    launch_dye_flags_begin(s, side);
     if (!s.ref) cudaMemsetAsync(s.redu + REDU_SPEED, 0, sizeof(unsigned int), side);
     launch_clear_splats(s, side);
+  } else {
+    launch_dye_flags_begin(s, st);
   }
   // the wave substep comes first and the advection reads its result
   // (BloodDropEngine.ts:1886-1912)
@@ -303,14 +305,9 @@ static void enqueue_step_body(dob_ctx* ctx, DevState& s, cudaStream_t st, float*
     } else if (!s.ref && stage == DOB_STAGE_CONC_PREDICT) {
       // closed box: the predictor brackets its taps for the resolve, which
       // then traces only the forward sample; both skip clear water
-      launch_conc_predict(s, st, true, true, side != nullptr);
+      launch_conc_predict(s, st, true, true);
     } else if (!s.ref && stage == DOB_STAGE_CONC_RESOLVE) {
-      launch_dye_resolve_lim(s, st, side != nullptr);
-      std::swap(s.conc, s.conc2);
-    } else if (side && stage == DOB_STAGE_CONC_PREDICT) {
-      launch_conc_predict(s, st, false, true, true);
-    } else if (side && stage == DOB_STAGE_CONC_RESOLVE) {
-      launch_conc_resolve(s, st, true, true);
+      launch_dye_resolve_lim(s, st, true);
       std::swap(s.conc, s.conc2);
     } else {
       enqueue_stage(ctx, s, stage, st, true);
@@ -623,7 +620,8 @@ dob_status dob_create(const dob_config* cfg, dob_ctx** out) {
   {
     const size_t nb = dye_brick_count(s.gc) * sizeof(uint32_t);
     A((void**)&s.cbrickA, nb); A((void**)&s.cbrickB, nb); A((void**)&s.sbrick, nb);
-    if (s.ref) A((void**)&s.pbrick, nb);
+    A((void**)&s.pbrick, nb); A((void**)&s.pold, nb); A((void**)&s.cold, nb);
+    if (s.ref) { A((void**)&s.hbrickA, nb); A((void**)&s.hbrickB, nb); }
   }
   if (!s.ref) A(&s.lim, Nc * 2 * dsb);
   A((void**)&s.splatI, Nc * 4); A((void**)&s.splatL, Nc * 4);
@@ -780,10 +778,10 @@ dob_status dob_reset(dob_ctx* ctx) {
   CK(cudaMemsetAsync(s.conc2, 0, Nc * nch * dsb, ctx->stream));
   if (s.cbrickA) {  // clear water everywhere
     const size_t nb = dye_brick_count(s.gc) * sizeof(uint32_t);
-    CK(cudaMemsetAsync(s.cbrickA, 0, nb, ctx->stream));
-    CK(cudaMemsetAsync(s.cbrickB, 0, nb, ctx->stream));
+    for (uint32_t* f : {s.cbrickA, s.cbrickB, s.hbrickA, s.hbrickB})
+      if (f) CK(cudaMemsetAsync(f, 0, nb, ctx->stream));
     CK(cudaMemsetAsync(s.sbrick, 0, nb, ctx->stream));  // the splat accumulators are zeroed below
-    if (s.pbrick) CK(cudaMemsetAsync(s.pbrick, 0, nb, ctx->stream));
+    CK(cudaMemsetAsync(s.pbrick, 1, nb, ctx->stream));  // the closed box's bracket is not cleared
   }
   CK(cudaMemsetAsync(s.pred, 0, Nc * dsb, ctx->stream));
   CK(cudaMemsetAsync(s.splatI, 0, Nc * 4, ctx->stream));
@@ -958,7 +956,7 @@ dob_status dob_set_field(dob_ctx* ctx, int field, const void* host, size_t bytes
   if (read_only || !field_desc(ctx, field, &f))
     return fail(ctx, DOB_EINVAL, "dob_set_field", "unknown or read-only field");
   if (bytes != f.count * 4) return fail(ctx, DOB_EINVAL, "dob_set_field", "byte count does not match the field");
-  if (field == DOB_FIELD_CONC) {
+  if (field == DOB_FIELD_CONC || field == DOB_FIELD_CONC_PRED) {
     dob_status bs = dye_bricks_unknown(ctx);
     if (bs != DOB_OK) return bs;
   }

@@ -38,6 +38,20 @@ __host__ __device__ __forceinline__ size_t rb_index(const Grid& d, int x, int y,
   return (size_t)((x + y + z) & 1) * half + ((size_t)z * d.ny + y) * (size_t)(d.nx >> 1) + (size_t)(x >> 1);
 }
 
+// 8x8x8 bricks of the dye grid, one uint32 flag each (k_fluid.cu)
+constexpr int kDyeBrick = 8;
+__host__ __device__ __forceinline__ Grid brick_grid(const Grid& gc) {
+  return Grid{(gc.nx + kDyeBrick - 1) / kDyeBrick, (gc.ny + kDyeBrick - 1) / kDyeBrick,
+              (gc.nz + kDyeBrick - 1) / kDyeBrick};
+}
+__device__ __forceinline__ size_t brick_of(const Grid& gc, int x, int y, int z) {
+  return brick_grid(gc).at(x / kDyeBrick, y / kDyeBrick, z / kDyeBrick);
+}
+// Whether the voxel's brick may hold anything but +0 (no flags: it may).
+__device__ __forceinline__ bool brick_held(const Grid& gc, const uint32_t* flags, int x, int y, int z) {
+  return !flags || __ldg(flags + brick_of(gc, x, y, z)) != 0u;
+}
+
 struct DevState {
   Grid g;    // velocity / pressure grid
   Grid gc;   // dye grid
@@ -58,12 +72,14 @@ struct DevState {
   float* parcels;
   uint32_t cap;
   // sparse dye bricks (k_fluid.cu): per 8x8x8 brick of the dye grid,
-  // whether the predictor (reference mode) / a dye buffer (its lysed
-  // channel in reference mode) holds a nonzero value; concA and concB are
-  // the buffers cbrickA and cbrickB belong to (conc and conc2 swap every
-  // step, the flags stay with their buffer; other dye arrays have none)
+  // whether the predictor's arrays (pbrick) / a dye buffer (cbrick: its lysed
+  // channel in reference mode; hbrick, reference mode: any channel) may hold
+  // a value that is not +0; concA and concB are the buffers the A and B flags
+  // belong to (conc and conc2 swap every step, the flags stay with their
+  // buffer; other dye arrays have none).  pold, cold: pbrick and the written
+  // dye buffer's flags as they were before the current step.
   const void *concA, *concB;
-  uint32_t *cbrickA, *cbrickB, *pbrick;
+  uint32_t *cbrickA, *cbrickB, *hbrickA, *hbrickB, *pbrick, *pold, *cold;
   // per 8x8x8 brick of the dye grid, whether the splat accumulators may
   // hold a nonzero sum there (set by every splat, cleared with the bricks)
   uint32_t* sbrick;
@@ -282,7 +298,8 @@ void launch_init_vel(const DevState& s, cudaStream_t st);
 void launch_advect_mac(const DevState& s, cudaStream_t st);
 void launch_mac_to_center(const DevState& s, cudaStream_t st);
 void launch_curl(const DevState& s, cudaStream_t st);
-void launch_casson(const DevState& s, cudaStream_t st);
+// sparse (inside a step, reference mode): clear water's dye is not read
+void launch_casson(const DevState& s, cudaStream_t st, bool sparse = false);
 void launch_mac_rhs(const DevState& s, cudaStream_t st);
 void launch_project(const DevState& s, cudaStream_t st);
 // ---- the 512x512 wave solver (k_wave.cu) -------------------------------------------------
@@ -318,19 +335,21 @@ void launch_project_center_ref(const DevState& s, cudaStream_t st);
 // by the projection's s.redu[REDU_SPEED] in the closed box): skip the
 // blocks the dye-brick flags show to be clear water (same results).  The
 // resolves always maintain the flags of the dye buffer they write.
-// cleared: launch_dye_flags_clear has cleared the flags that the predictor
-// and the resolve of this step write (else they clear them themselves).
-void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket = false, bool sparse = false,
-                         bool cleared = false);
-void launch_dye_resolve_lim(const DevState& s, cudaStream_t st, bool cleared = false);
-void launch_dye_flags_clear(const DevState& s, cudaStream_t st);
+// launch_dye_flags_begin goes before them (once a step, in any order with the
+// stages up to the projection): it keeps the old flags of what they write.
+void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket = false, bool sparse = false);
+void launch_dye_resolve_lim(const DevState& s, cudaStream_t st, bool sparse = false);
+void launch_dye_flags_begin(const DevState& s, cudaStream_t st);
+// flags of all channels of one of the context's dye buffers (null for others)
+uint32_t* held_flags_of(const DevState& s, const void* conc);
 // dye written from outside the step (injection, field I/O, snapshots, the
-// tape): every brick of both dye buffers may hold dye until the next resolve
+// tape): every brick of both dye buffers and of the predictor's arrays may
+// hold something until it is rewritten
 void launch_dye_bricks_unknown(const DevState& s, cudaStream_t st);
 // zero the splat accumulators: only the bricks a splat has marked (the
 // others hold zeros already), then clear their marks
 void launch_clear_splats(const DevState& s, cudaStream_t st);
-void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse = false, bool cleared = false);
+void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse = false);
 // number of 8x8x8 dye bricks (one uint32 flag each)
 size_t dye_brick_count(const Grid& gc);
 

@@ -306,6 +306,66 @@ __global__ void __launch_bounds__(256) k_curl(Grid g, const typename Vec4Of<VS>:
   st4(curl + i, make_float4(om.x, om.y, om.z, mag));
 }
 
+// ---- sparse dye bricks ---------------------------------------------------------------------
+// Most of the dye grid is clear water.  Flags per 8x8x8 brick of it say where
+// an array may hold anything but +0: for the predictor's arrays (pbrick: the
+// prediction and, in the closed box, its bracket) and for each dye buffer
+// (held_flags_of: all channels; cbrick in reference mode the lysed channel
+// alone, .y, the only one the predictor reads).  Inside a step
+//   - the predictor skips a block whose departure points can only reach bricks
+//     without (lysed) dye: its result there is exactly +0;
+//   - the reference resolve skips the voxels of a block that sees no predictor
+//     value within one voxel and no splat, and the box's those whose bracket is
+//     two zeros: the result there is exactly +0;
+//   - the zeros of a skipped voxel are stored only where the array's last
+//     contents (pold, cold: the flags before this step) may not be zero already;
+//   - the reference resolve reads the splat sums, the Casson stages the dye and
+//     the box's resolve the bracket only where the flags say there may be any.
+// So clear water costs flag reads, not the 5 to 9 words per voxel these stages
+// touch: reference Casson 54 -> 34 us and resolve 73 -> 58 us at 96x128x96 (dye
+// 192x256x192), the box's predictor and resolve 75 -> 47 and 44 -> 24 us at
+// 192x256x192.  (Casson of the box reads the dye everywhere: 76 us with the
+// flags, 78 without, all of it hidden behind the velocity's traffic.)  Flags are plain stores of 1 (a race between writers of the same
+// value is harmless); launch_dye_flags_begin clears them.
+// |centre velocity| per axis inside a step: the projection clamps the faces
+// to +-2 (fluid.ts:908) and the centre is their mean (with a margin)
+constexpr float kDyeSpeedBound = 2.0f * 1.0001f;
+constexpr int kDyeResolveZ = 4;  // voxels per thread along z in the sparse predictor and resolves (divides kDyeBrick)
+__device__ __forceinline__ void mark_brick(const Grid& gc, uint32_t* flags, int x, int y, int z) {
+  flags[brick_of(gc, x, y, z)] = 1u;
+}
+// Whether any brick overlapping the voxels [x0, x1] x [y0, y1] x [z0, z1]
+// (clamped to the grid) is flagged (arguments uniform over the block; every
+// thread must call it).
+__device__ __forceinline__ bool any_brick(const Grid& gc, const uint32_t* flags, int x0, int x1, int y0, int y1,
+                                          int z0, int z1) {
+  __shared__ int any;
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  if (tid == 0) any = 0;
+  __syncthreads();
+  x0 = max(x0, 0); x1 = min(x1, gc.nx - 1);
+  y0 = max(y0, 0); y1 = min(y1, gc.ny - 1);
+  z0 = max(z0, 0); z1 = min(z1, gc.nz - 1);
+  const Grid b = brick_grid(gc);
+  const int bx0 = x0 / kDyeBrick, by0 = y0 / kDyeBrick, bz0 = z0 / kDyeBrick;
+  const int nbx = x1 / kDyeBrick - bx0 + 1, nby = y1 / kDyeBrick - by0 + 1, nbz = z1 / kDyeBrick - bz0 + 1;
+  const int count = nbx * nby * nbz;
+  for (int k = tid; k < count; k += blockDim.x * blockDim.y) {
+    const int ix = k % nbx, iy = (k / nbx) % nby, iz = k / (nbx * nby);
+    if (__ldg(flags + b.at(bx0 + ix, by0 + iy, bz0 + iz))) any = 1;
+  }
+  __syncthreads();
+  return any != 0;
+}
+// The same for the block's voxels (x and y from the block index, planes
+// zlo..zhi), widened by rx, ry, rz voxels per axis.
+__device__ __forceinline__ bool block_any_brick(const Grid& gc, const uint32_t* flags, int rx, int ry, int rz,
+                                                int zlo, int zhi) {
+  const int x = (int)(blockIdx.x * blockDim.x), y = (int)(blockIdx.y * blockDim.y);
+  return any_brick(gc, flags, x - rx, x + (int)blockDim.x - 1 + rx, y - ry, y + (int)blockDim.y - 1 + ry, zlo - rz,
+                   zhi + rz);
+}
+
 // ---- FLUID_CASSON_FORCES (fluid.ts:377-511) ------------------------------------------------
 template <class VS>
 __device__ __forceinline__ dob_v3 ldmac(const Grid& g, const VS* u, const VS* v, const VS* w, int x, int y, int z) {
@@ -340,8 +400,21 @@ __global__ void __launch_bounds__(256) k_casson(Grid g, Grid gc, const StepParam
                                                 const VS* __restrict__ w,
                                                 const typename Vec4Of<VS>::type* __restrict__ curl,
                                                 const typename Vec4Of<DS>::type* __restrict__ conc4,
-                                                const DS* __restrict__ dye, VS* __restrict__ uo, VS* __restrict__ vo,
-                                                VS* __restrict__ wo) {
+                                                const DS* __restrict__ dye, const uint32_t* __restrict__ held,
+                                                VS* __restrict__ uo, VS* __restrict__ vo, VS* __restrict__ wo) {
+  // held (reference mode inside a step): the dye's flags.  The cell's two
+  // samples, at its centre and on its upper y face, tap dye voxels r x - 1 to
+  // r (x + 1) per axis (r dye cells per cell); one more for the rounding of
+  // the texel and 1/1000 of the axis, by which the face sample is clamped into
+  // the domain.  Over clear water both are +0 and not formed.
+  bool dyed = true;
+  if (held) {
+    const int r = gc.nx / g.nx;
+    const int x0 = (int)(blockIdx.x * blockDim.x) * r, y0 = (int)(blockIdx.y * blockDim.y) * r, z0 = (int)blockIdx.z * r;
+    const int mx = 2 + gc.nx / 1000, my = 2 + gc.ny / 1000, mz = 2 + gc.nz / 1000;
+    dyed = any_brick(gc, held, x0 - mx, x0 + (int)blockDim.x * r + mx, y0 - my, y0 + (int)blockDim.y * r + my, z0 - mz,
+                     z0 + r + mz);
+  }
   CELL_INDEX
   const StepParams& P = *Pp;
   const Recip3 dims = grid_recip(g);
@@ -354,7 +427,7 @@ __global__ void __launch_bounds__(256) k_casson(Grid g, Grid gc, const StepParam
   const dob_v3 du = mXp - mXn, dv = mYp - mYn, dw = mZp - mZn;
   const dob_v3 lapMac = (mXp + mXn + mYp + mYn + mZp + mZn) - 6.0f * mac;
   if (ref) {
-    const dob_v3 concCell = sample_conc_rg<DS>(gc, conc4, uvwCell);
+    const dob_v3 concCell = dyed ? sample_conc_rg<DS>(gc, conc4, uvwCell) : v3(0.0f, 0.0f, 0.0f);
     const float cRbc = dob_clampf(concCell.x, 0.0f, 1.5f);
     const float cassonScale = P.U[58];
     const float sqrtMuInf = dob_sqrt(0.00010f * (1.0f + 1.35f * cRbc));
@@ -378,7 +451,7 @@ __global__ void __launch_bounds__(256) k_casson(Grid g, Grid gc, const StepParam
       const float vcZ = 0.5f * (vc0.z + vort_conf(g, curl, x, y, min(z + 1, g.nz - 1), vcs).z);
       mac = mac + v3(vcX, vcY, vcZ) * dtv;
     }
-    if (flags & DOB_PHYS_BUOYANCY) {
+    if (dyed && (flags & DOB_PHYS_BUOYANCY)) {  // no dye: buoyDensity = 0
       const dob_v3 uvwFaceY = v3((float)x + 0.5f, (float)y + 1.0f, (float)z + 0.5f) / dims;
       const dob_v3 cf = sample_conc_rg<DS>(gc, conc4, clamp3(uvwFaceY, 0.001f, 0.999f));
       const float buoyDensity = 1.24f * cf.x + 0.26f * cf.y;
@@ -544,53 +617,6 @@ __global__ void __launch_bounds__(256) k_divergence(Grid g, int ref, const VS* _
   if (maxbits) block_max_atomic(m, maxbits);
 }
 
-// ---- sparse dye bricks (reference mode) ------------------------------------------------------
-// Most of the 192x256x192 dye grid is clear water.  Per 8x8x8 brick of the
-// dye grid the predictor records whether any of its values is nonzero, and
-// the resolve whether any lysed value (.y, the only channel the predictor
-// reads) of its output is.  Inside a step the predictor skips a block whose
-// departure points can only reach bricks without lysed dye (its result
-// there is exactly +0), and the resolve skips the voxels of a block that
-// sees no predictor value within one voxel and no splat (its early-out
-// writes exactly zeros there).  Flags are plain stores of 1 (a race between
-// writers of the same value is harmless); the launchers clear them first.
-constexpr int kDyeBrick = 8;
-// |centre velocity| per axis inside a step: the projection clamps the faces
-// to +-2 (fluid.ts:908) and the centre is their mean (with a margin)
-constexpr float kDyeSpeedBound = 2.0f * 1.0001f;
-constexpr int kDyeResolveZ = 4;  // voxels per thread along z in the reference-mode resolve
-__host__ __device__ __forceinline__ Grid brick_grid(const Grid& gc) {
-  return Grid{(gc.nx + kDyeBrick - 1) / kDyeBrick, (gc.ny + kDyeBrick - 1) / kDyeBrick,
-              (gc.nz + kDyeBrick - 1) / kDyeBrick};
-}
-__device__ __forceinline__ void mark_brick(const Grid& gc, uint32_t* flags, int x, int y, int z) {
-  flags[brick_grid(gc).at(x / kDyeBrick, y / kDyeBrick, z / kDyeBrick)] = 1u;
-}
-// Whether any brick overlapping the block's voxels (x and y from the block
-// index, planes zlo..zhi), widened by rx, ry, rz voxels per axis, is flagged
-// (block-uniform; every thread must call it).
-__device__ __forceinline__ bool block_any_brick(const Grid& gc, const uint32_t* flags, int rx, int ry, int rz,
-                                                int zlo, int zhi) {
-  __shared__ int any;
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-  if (tid == 0) any = 0;
-  __syncthreads();
-  const int x0 = max((int)(blockIdx.x * blockDim.x) - rx, 0);
-  const int x1 = min((int)(blockIdx.x * blockDim.x + blockDim.x) - 1 + rx, gc.nx - 1);
-  const int y0 = max((int)(blockIdx.y * blockDim.y) - ry, 0);
-  const int y1 = min((int)(blockIdx.y * blockDim.y + blockDim.y) - 1 + ry, gc.ny - 1);
-  const int z0 = max(zlo - rz, 0), z1 = min(zhi + rz, gc.nz - 1);
-  const Grid b = brick_grid(gc);
-  const int bx0 = x0 / kDyeBrick, by0 = y0 / kDyeBrick, bz0 = z0 / kDyeBrick;
-  const int nbx = x1 / kDyeBrick - bx0 + 1, nby = y1 / kDyeBrick - by0 + 1, nbz = z1 / kDyeBrick - bz0 + 1;
-  const int count = nbx * nby * nbz;
-  for (int k = tid; k < count; k += blockDim.x * blockDim.y) {
-    const int ix = k % nbx, iy = (k / nbx) % nby, iz = k / (nbx * nby);
-    if (__ldg(flags + b.at(bx0 + ix, by0 + iy, bz0 + iz))) any = 1;
-  }
-  __syncthreads();
-  return any != 0;
-}
 // The predictor's reach: RK2 departures move at most `speed` dt per axis in
 // world units, plus one voxel for the interpolation's taps (a reach of the
 // whole grid or more, or a non-finite speed, covers the whole grid).
@@ -626,7 +652,7 @@ __device__ __forceinline__ void predict_cell(const Grid& gc, const Grid& g, cons
     if (speed2 < 2.5e-5f) {
       const float pv = ld4(conc4 + i).y;
       stf(pred + i, pv);
-      if (pbrick && pv != 0.0f) mark_brick(gc, pbrick, x, y, z);
+      if (pbrick && __float_as_uint(pv) != 0u) mark_brick(gc, pbrick, x, y, z);
       return;
     }
     dob_v3 back;
@@ -640,7 +666,7 @@ __device__ __forceinline__ void predict_cell(const Grid& gc, const Grid& g, cons
     const Taps t = make_taps_in(gc, back.x, back.y, back.z);
     const float pv = lerp8xn<2>(t, conc4).y;
     stf(pred + i, pv);
-    if (pbrick && pv != 0.0f) mark_brick(gc, pbrick, x, y, z);
+    if (pbrick && __float_as_uint(pv) != 0u) mark_brick(gc, pbrick, x, y, z);
   } else {
     const dob_v3 v0 = gc.nx == g.nx ? center_at_cell(g, cen, uvw, x, y, z, i) : sample_center(g, cen, uvw);
     const dob_v3 mid = clamp3(uvw - (0.5f * (v0 * dtv)) / dom, 0.001f, 0.999f);
@@ -650,9 +676,12 @@ __device__ __forceinline__ void predict_cell(const Grid& gc, const Grid& g, cons
     if (lim) {  // also the limiter's bracket for k_dye_resolve_lim
       float c[8];
       load8(tb, dye, c);
-      stf(pred + i, tri(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], tb));
-      stf(lim + 2 * i, min8(c));
-      stf(lim + 2 * i + 1, max8(c));
+      const float pv = tri(c[0], c[1], c[2], c[3], c[4], c[5], c[6], c[7], tb), lo = min8(c), hi = max8(c);
+      stf(pred + i, pv);
+      stf(lim + 2 * i, lo);
+      stf(lim + 2 * i + 1, hi);
+      if (pbrick && (__float_as_uint(pv) | __float_as_uint(lo) | __float_as_uint(hi)) != 0u)
+        mark_brick(gc, pbrick, x, y, z);
     } else {
       stf(pred + i, lerp8(tb, dye));
     }
@@ -660,15 +689,15 @@ __device__ __forceinline__ void predict_cell(const Grid& gc, const Grid& g, cons
 }
 
 // ZP voxels per thread along z (grid z = nz / ZP): with the brick flags
-// (reference mode inside a step, ZP = kDyeResolveZ) one reach test serves
-// ZP planes; the closed box runs one voxel per thread.
+// (inside a step, ZP = kDyeResolveZ) one reach test serves ZP planes;
+// without them one voxel per thread.
 template <class VS, class DS, int ZP>
 __global__ void __launch_bounds__(256, ZP == 1 ? 8 : 4) k_conc_predict(Grid gc, Grid g, const StepParams* __restrict__ Pp, int ref,
                                                       const typename Vec4Of<VS>::type* __restrict__ cen,
                                                       const typename Vec4Of<DS>::type* __restrict__ conc4,
                                                       const DS* __restrict__ dye, DS* __restrict__ pred,
                                                       DS* __restrict__ lim, const uint32_t* __restrict__ cbrick,
-                                                      uint32_t* __restrict__ pbrick,
+                                                      uint32_t* __restrict__ pbrick, const uint32_t* __restrict__ pold,
                                                       const unsigned int* __restrict__ speedbits) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
@@ -684,7 +713,7 @@ __global__ void __launch_bounds__(256, ZP == 1 ? 8 : 4) k_conc_predict(Grid gc, 
   if (cbrick) {
     const float speed = speedbits ? __uint_as_float(*speedbits) * 1.0001f : kDyeSpeedBound;
     if (!block_reaches_dye(gc, P, cbrick, speed, z0, z1 - 1)) {
-      if (x < gc.nx && y < gc.ny)
+      if (x < gc.nx && y < gc.ny && brick_held(gc, pold, x, y, z0))
         for (int z = z0; z < z1; ++z) {
           const size_t i = gc.at(x, y, z);
           stf(pred + i, 0.0f);
@@ -720,7 +749,8 @@ __device__ __forceinline__ void resolve_ref_cell(const Grid& gc, const Grid& g, 
                                                  const DS* __restrict__ pred, const uint32_t* __restrict__ splatI,
                                                  const uint32_t* __restrict__ splatL,
                                                  typename Vec4Of<DS>::type* __restrict__ out,
-                                                 uint32_t* __restrict__ cbrick_out, int x, int y, int z) {
+                                                 uint32_t* __restrict__ cbrick_out, uint32_t* __restrict__ held_out,
+                                                 int x, int y, int z) {
   const size_t i = gc.at(x, y, z);
   const dob_v3 dims = v3((float)gc.nx, (float)gc.ny, (float)gc.nz);
   const Recip3 dimr = grid_recip(gc);
@@ -830,6 +860,8 @@ __device__ __forceinline__ void resolve_ref_cell(const Grid& gc, const Grid& g, 
   }
   st4(out + i, make_float4(cIntact, cLysed, vOx, cBed));
   if (cLysed != 0.0f) mark_brick(gc, cbrick_out, x, y, z);
+  if ((__float_as_uint(cIntact) | __float_as_uint(cLysed) | __float_as_uint(vOx) | __float_as_uint(cBed)) != 0u)
+    mark_brick(gc, held_out, x, y, z);
 }
 
 // Each thread resolves kDyeResolveZ voxels along z: their splat sums are
@@ -845,16 +877,21 @@ __global__ void __launch_bounds__(256, 3) k_conc_resolve_ref(Grid gc, Grid g, co
                                                           const uint32_t* __restrict__ splatI,
                                                           const uint32_t* __restrict__ splatL,
                                                           typename Vec4Of<DS>::type* __restrict__ out,
+                                                          const uint32_t* __restrict__ sbrick,
                                                           const uint32_t* __restrict__ pbrick,
-                                                          uint32_t* __restrict__ cbrick_out) {
+                                                          const uint32_t* __restrict__ cold,
+                                                          uint32_t* __restrict__ cbrick_out,
+                                                          uint32_t* __restrict__ held_out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
   const int z0 = blockIdx.z * kDyeResolveZ;
   const bool inside = x < gc.nx && y < gc.ny;
+  const bool splats = inside && brick_held(gc, sbrick, x, y, z0);
+  const bool held = inside && brick_held(gc, cold, x, y, z0);
   uint32_t rI[kDyeResolveZ], rL[kDyeResolveZ];
 #pragma unroll
   for (int k = 0; k < kDyeResolveZ; ++k) {
-    const bool ok = inside && z0 + k < gc.nz;
+    const bool ok = splats && z0 + k < gc.nz;
     const size_t i = ok ? gc.at(x, y, z0 + k) : 0;
     rI[k] = ok ? __ldg(splatI + i) : 0u;
     rL[k] = ok ? __ldg(splatL + i) : 0u;
@@ -871,16 +908,16 @@ __global__ void __launch_bounds__(256, 3) k_conc_resolve_ref(Grid gc, Grid g, co
     if (z >= gc.nz) break;
     // the boundary shell, and clear water's early-out (every predictor tap
     // +0, so oct0 = oct1 = 0 below) outside the floor zone
-    if (shellXY || z == 0 || z >= gc.nz - 1 || (clear && !inFloorZone && rI[k] == 0u && rL[k] == 0u))
-      st4(out + gc.at(x, y, z), make_float4(0.f, 0.f, 0.f, 0.f));
-    else
+    if (!(shellXY || z == 0 || z >= gc.nz - 1 || (clear && !inFloorZone && rI[k] == 0u && rL[k] == 0u)))
       need |= 1u << k;
+    else if (held)
+      st4(out + gc.at(x, y, z), make_float4(0.f, 0.f, 0.f, 0.f));
   }
   const StepParams& P = *Pp;
   while (need) {
     const int k = __ffs(need) - 1;
     need &= need - 1u;
-    resolve_ref_cell<VS, DS>(gc, g, P, cen, conc, pred, splatI, splatL, out, cbrick_out, x, y, z0 + k);
+    resolve_ref_cell<VS, DS>(gc, g, P, cen, conc, pred, splatI, splatL, out, cbrick_out, held_out, x, y, z0 + k);
   }
 }
 
@@ -921,15 +958,11 @@ __global__ void __launch_bounds__(256) k_dye_resolve_box(Grid gc, Grid g, const 
 // cbrick_out (the flags of `out`): a brick is marked when it receives a
 // value whose bits are not those of +0.
 template <class VS, class DS>
-__global__ void __launch_bounds__(256, 8) k_dye_resolve_lim(Grid gc, Grid g, const StepParams* __restrict__ Pp,
-                                                         const typename Vec4Of<VS>::type* __restrict__ cen,
-                                                         const DS* __restrict__ dye, const DS* __restrict__ pred,
-                                                         const DS* __restrict__ lim, DS* __restrict__ out,
-                                                         uint32_t* __restrict__ cbrick_out) {
-  const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int z = blockIdx.z;
-  if (x >= gc.nx || y >= gc.ny) return;
+__device__ __forceinline__ void resolve_lim_cell(const Grid& gc, const Grid& g, const StepParams& P,
+                                                 const typename Vec4Of<VS>::type* __restrict__ cen,
+                                                 const DS* __restrict__ dye, const DS* __restrict__ pred,
+                                                 const DS* __restrict__ lim, DS* __restrict__ out,
+                                                 uint32_t* __restrict__ cbrick_out, int x, int y, int z) {
   const size_t i = gc.at(x, y, z);
   // A bracket of two zeros clamps every correction to its upper end: min(max(g,
   // lo), hi) is hi whenever lo and hi are zeros of either sign (max gives g > 0
@@ -940,7 +973,6 @@ __global__ void __launch_bounds__(256, 8) k_dye_resolve_lim(Grid gc, Grid g, con
     if (cbrick_out && __float_as_uint(hi) != 0u) mark_brick(gc, cbrick_out, x, y, z);
     return;
   }
-  const StepParams& P = *Pp;
   const float dtv = P.dt;
   const Recip3 dom = dom_recip(P);
   const dob_v3 uvw = (v3((float)x, (float)y, (float)z) + v3(0.5f, 0.5f, 0.5f)) /
@@ -956,8 +988,41 @@ __global__ void __launch_bounds__(256, 8) k_dye_resolve_lim(Grid gc, Grid g, con
   stf(out + i, r);
   if (cbrick_out && __float_as_uint(r) != 0u) mark_brick(gc, cbrick_out, x, y, z);
 }
+// ZP voxels per thread along z.  pbrick (inside a step): where the
+// predictor left its arrays at +0, the bracket is not read, and the zero is
+// stored only where cold says that `out` may hold something else.
+template <class VS, class DS, int ZP>
+__global__ void __launch_bounds__(256, ZP == 1 ? 8 : 5) k_dye_resolve_lim(Grid gc, Grid g, const StepParams* __restrict__ Pp,
+                                                         const typename Vec4Of<VS>::type* __restrict__ cen,
+                                                         const DS* __restrict__ dye, const DS* __restrict__ pred,
+                                                         const DS* __restrict__ lim, DS* __restrict__ out,
+                                                         const uint32_t* __restrict__ pbrick,
+                                                         const uint32_t* __restrict__ cold,
+                                                         uint32_t* __restrict__ cbrick_out) {
+  const int x = blockIdx.x * blockDim.x + threadIdx.x;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int z0 = blockIdx.z * ZP, z1 = min(z0 + ZP, gc.nz);
+  if (x >= gc.nx || y >= gc.ny) return;
+  if (!brick_held(gc, pbrick, x, y, z0)) {
+    if (brick_held(gc, cold, x, y, z0))
+      for (int z = z0; z < z1; ++z) stf(out + gc.at(x, y, z), 0.0f);
+    return;
+  }
+#pragma unroll 1
+  for (int z = z0; z < z1; ++z) resolve_lim_cell<VS, DS>(gc, g, *Pp, cen, dye, pred, lim, out, cbrick_out, x, y, z);
+}
 
 // ---- host launchers ------------------------------------------------------------------------------
+// the dye-brick flags of one of the context's two dye buffers (none for
+// other dye arrays, such as the adjoint's tape): the channel the predictor
+// reads, and all channels
+static uint32_t* brick_flags_of(const DevState& s, const void* conc) {
+  return conc == s.concA ? s.cbrickA : conc == s.concB ? s.cbrickB : nullptr;
+}
+uint32_t* held_flags_of(const DevState& s, const void* conc) {
+  if (!s.ref) return brick_flags_of(s, conc);
+  return conc == s.concA ? s.hbrickA : conc == s.concB ? s.hbrickB : nullptr;
+}
 static inline dim3 cell_grid(const Grid& g) { return dim3((g.nx + 31) / 32, (g.ny + 7) / 8, g.nz); }
 static inline dim3 cell_block() { return dim3(32, 8, 1); }
 
@@ -998,12 +1063,16 @@ void launch_curl(const DevState& s, cudaStream_t st) {
   });
 }
 
-void launch_casson(const DevState& s, cudaStream_t st) {
+void launch_casson(const DevState& s, cudaStream_t st, bool sparse) {
+  // the samples' reach is worked out for whole dye cells per velocity cell
+  const int r = s.gc.nx / s.g.nx;
+  const bool whole = s.gc.nx == r * s.g.nx && s.gc.ny == r * s.g.ny && s.gc.nz == r * s.g.nz;
+  const uint32_t* held = sparse && s.ref && whole ? held_flags_of(s, s.conc) : nullptr;
   DOB_VEL_DISPATCH(s.prec, {
     k_casson<VS, DS><<<cell_grid(s.g), cell_block(), 0, st>>>(
         s.g, s.gc, s.params, s.ref, s.flags, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w,
         (const typename Vec4Of<VS>::type*)s.curl, (const typename Vec4Of<DS>::type*)s.conc, (const DS*)s.conc,
-        (VS*)s.u2, (VS*)s.v2, (VS*)s.w2);
+        held, (VS*)s.u2, (VS*)s.v2, (VS*)s.w2);
   });
 }
 
@@ -1040,68 +1109,92 @@ void launch_divergence(const DevState& s, float* out, float scale, unsigned int*
   });
 }
 
-// the dye-brick flags of one of the context's two dye buffers (none for
-// other dye arrays, such as the adjoint's tape)
-static uint32_t* brick_flags_of(const DevState& s, const void* conc) {
-  return conc == s.concA ? s.cbrickA : conc == s.concB ? s.cbrickB : nullptr;
-}
 void launch_dye_bricks_unknown(const DevState& s, cudaStream_t st) {
   const size_t nb = brick_grid(s.gc).n() * sizeof(uint32_t);
-  if (s.cbrickA) cudaMemsetAsync(s.cbrickA, 1, nb, st);
-  if (s.cbrickB) cudaMemsetAsync(s.cbrickB, 1, nb, st);
+  for (uint32_t* f : {s.cbrickA, s.cbrickB, s.hbrickA, s.hbrickB, s.pbrick})
+    if (f) cudaMemsetAsync(f, 1, nb, st);
 }
 size_t dye_brick_count(const Grid& gc) { return brick_grid(gc).n(); }
 
-void launch_dye_flags_clear(const DevState& s, cudaStream_t st) {
-  const size_t nb = brick_grid(s.gc).n() * sizeof(uint32_t);
-  if (s.ref && s.pbrick) cudaMemsetAsync(s.pbrick, 0, nb, st);
-  if (uint32_t* cb = brick_flags_of(s, s.conc2)) cudaMemsetAsync(cb, 0, nb, st);
+// Old flags kept (pold, cold), the flags of what this step writes cleared.
+__global__ void __launch_bounds__(256) k_dye_flags_begin(size_t nb, uint32_t* __restrict__ pbrick,
+                                                         uint32_t* __restrict__ pold, uint32_t* __restrict__ held_out,
+                                                         uint32_t* __restrict__ cold,
+                                                         uint32_t* __restrict__ cbrick_out) {
+  const size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (b >= nb) return;
+  pold[b] = pbrick[b];
+  pbrick[b] = 0u;
+  cold[b] = held_out[b];
+  held_out[b] = 0u;
+  if (cbrick_out != held_out) cbrick_out[b] = 0u;
+}
+void launch_dye_flags_begin(const DevState& s, cudaStream_t st) {
+  const size_t nb = brick_grid(s.gc).n();
+  k_dye_flags_begin<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(nb, s.pbrick, s.pold, held_flags_of(s, s.conc2),
+                                                                 s.cold, brick_flags_of(s, s.conc2));
 }
 
-void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket, bool sparse, bool cleared) {
-  uint32_t* pb = s.ref ? s.pbrick : nullptr;
-  if (pb && !cleared) cudaMemsetAsync(pb, 0, brick_grid(s.gc).n() * sizeof(uint32_t), st);
+// The closed box's sparse predictor and resolve take kDyeResolveZ voxels per
+// thread where that still gives 8 blocks per SM (192x256x192: predictor 75 ->
+// 47 us, resolve 44 -> 24), else one (48x64x48: 9.5 and 7.5 us, 11.8 and 10.0
+// with four; 96x128x96: resolve 10.4, 12.5 with four).
+static bool sparse_planes(const DevState& s) {
+  const dim3 gr = cell_grid(s.gc);
+  return (size_t)gr.x * gr.y * gr.z >= (size_t)kDyeResolveZ * 8 * s.num_sms;
+}
+
+void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket, bool sparse) {
   const uint32_t* cb = sparse ? brick_flags_of(s, s.conc) : nullptr;
+  // outside a step the predictor's arrays (the tape's share the bracket)
+  // may then hold anything
+  if (!sparse && s.pbrick) cudaMemsetAsync(s.pbrick, 1, brick_grid(s.gc).n() * sizeof(uint32_t), st);
   DOB_VEL_DISPATCH(s.prec, {
-    if (cb && s.ref) {
+    auto run = [&](auto* k, int zp) {
       dim3 gr = cell_grid(s.gc);
-      gr.z = (s.gc.nz + kDyeResolveZ - 1) / kDyeResolveZ;
-      k_conc_predict<VS, DS, kDyeResolveZ><<<gr, cell_block(), 0, st>>>(
-          s.gc, s.g, s.params, s.ref, (const typename Vec4Of<VS>::type*)s.cen,
-          (const typename Vec4Of<DS>::type*)s.conc, (const DS*)s.conc, (DS*)s.pred, nullptr, cb, pb, nullptr);
-    } else {
+      gr.z = (s.gc.nz + zp - 1) / zp;
       // the closed box's bound on the centre velocity comes from the projection
-      k_conc_predict<VS, DS, 1><<<cell_grid(s.gc), cell_block(), 0, st>>>(
-          s.gc, s.g, s.params, s.ref, (const typename Vec4Of<VS>::type*)s.cen,
-          (const typename Vec4Of<DS>::type*)s.conc, (const DS*)s.conc, (DS*)s.pred,
-          bracket && !s.ref ? (DS*)s.lim : nullptr, cb, pb, cb ? s.redu + REDU_SPEED : nullptr);
-    }
+      k<<<gr, cell_block(), 0, st>>>(s.gc, s.g, s.params, s.ref, (const typename Vec4Of<VS>::type*)s.cen,
+                                     (const typename Vec4Of<DS>::type*)s.conc, (const DS*)s.conc, (DS*)s.pred,
+                                     bracket && !s.ref ? (DS*)s.lim : nullptr, cb, sparse ? s.pbrick : nullptr, s.pold,
+                                     cb && !s.ref ? s.redu + REDU_SPEED : nullptr);
+    };
+    if (cb && (s.ref || sparse_planes(s))) run(k_conc_predict<VS, DS, kDyeResolveZ>, kDyeResolveZ);
+    else run(k_conc_predict<VS, DS, 1>, 1);
   });
 }
 
-void launch_dye_resolve_lim(const DevState& s, cudaStream_t st, bool cleared) {
-  uint32_t* cb = brick_flags_of(s, s.conc2);
-  if (cb && !cleared) cudaMemsetAsync(cb, 0, brick_grid(s.gc).n() * sizeof(uint32_t), st);
+void launch_dye_resolve_lim(const DevState& s, cudaStream_t st, bool sparse) {
   DOB_VEL_DISPATCH(s.prec, {
-    k_dye_resolve_lim<VS, DS><<<cell_grid(s.gc), cell_block(), 0, st>>>(
-        s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const DS*)s.conc, (const DS*)s.pred,
-        (const DS*)s.lim, (DS*)s.conc2, cb);
+    auto run = [&](auto* k, int zp) {
+      dim3 gr = cell_grid(s.gc);
+      gr.z = (s.gc.nz + zp - 1) / zp;
+      k<<<gr, cell_block(), 0, st>>>(s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const DS*)s.conc,
+                                     (const DS*)s.pred, (const DS*)s.lim, (DS*)s.conc2, sparse ? s.pbrick : nullptr,
+                                     sparse ? s.cold : nullptr, brick_flags_of(s, s.conc2));
+    };
+    if (sparse && sparse_planes(s)) run(k_dye_resolve_lim<VS, DS, kDyeResolveZ>, kDyeResolveZ);
+    else run(k_dye_resolve_lim<VS, DS, 1>, 1);
   });
 }
 
-void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse, bool cleared) {
-  uint32_t* cb = brick_flags_of(s, s.conc2);
-  // reference mode: the resolve rewrites its output's flags; the closed box's
-  // tracing resolve does not, so its output's flags say "may hold dye"
-  if (cb && !cleared) cudaMemsetAsync(cb, s.ref ? 0 : 1, brick_grid(s.gc).n() * sizeof(uint32_t), st);
+void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse) {
+  uint32_t *cb = brick_flags_of(s, s.conc2), *hb = held_flags_of(s, s.conc2);
+  if (!sparse) {
+    // reference mode: the resolve rewrites its output's flags; the closed box's
+    // tracing resolve does not, so its output's flags say "may hold dye"
+    const size_t nb = brick_grid(s.gc).n() * sizeof(uint32_t);
+    for (uint32_t* f : {cb, hb})
+      if (f) cudaMemsetAsync(f, s.ref ? 0 : 1, nb, st);
+  }
   DOB_VEL_DISPATCH(s.prec, {
     if (s.ref) {
       dim3 gr = cell_grid(s.gc);
       gr.z = (s.gc.nz + kDyeResolveZ - 1) / kDyeResolveZ;
       k_conc_resolve_ref<VS, DS><<<gr, cell_block(), 0, st>>>(
           s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const typename Vec4Of<DS>::type*)s.conc,
-          (const DS*)s.pred, s.splatI, s.splatL, (typename Vec4Of<DS>::type*)s.conc2, sparse ? s.pbrick : nullptr,
-          cb);
+          (const DS*)s.pred, s.splatI, s.splatL, (typename Vec4Of<DS>::type*)s.conc2, s.sbrick,
+          sparse ? s.pbrick : nullptr, sparse ? s.cold : nullptr, cb, hb);
     } else {
       k_dye_resolve_box<VS, DS><<<cell_grid(s.gc), cell_block(), 0, st>>>(
           s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const DS*)s.conc, (const DS*)s.pred,
