@@ -621,6 +621,7 @@ dob_status dob_create(const dob_config* cfg, dob_ctx** out) {
     const size_t nb = dye_brick_count(s.gc) * sizeof(uint32_t);
     A((void**)&s.cbrickA, nb); A((void**)&s.cbrickB, nb); A((void**)&s.sbrick, nb);
     A((void**)&s.pbrick, nb); A((void**)&s.pold, nb); A((void**)&s.cold, nb);
+    A((void**)&s.dye_list, nb + 2 * sizeof(uint32_t));
     if (s.ref) { A((void**)&s.hbrickA, nb); A((void**)&s.hbrickB, nb); }
   }
   if (!s.ref) A(&s.lim, Nc * 2 * dsb);

@@ -80,6 +80,7 @@ struct DevState {
   // dye buffer's flags as they were before the current step.
   const void *concA, *concB;
   uint32_t *cbrickA, *cbrickB, *hbrickA, *hbrickB, *pbrick, *pold, *cold;
+  uint32_t* dye_list;            // counts of the predictor's and the resolve's list, the list (a brick's index each)
   // per 8x8x8 brick of the dye grid, whether the splat accumulators may
   // hold a nonzero sum there (set by every splat, cleared with the bricks)
   uint32_t* sbrick;

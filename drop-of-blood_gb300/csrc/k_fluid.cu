@@ -314,23 +314,22 @@ __global__ void __launch_bounds__(256) k_curl(Grid g, const typename Vec4Of<VS>:
 // alone, .y, the only one the predictor reads).  Inside a step
 //   - the predictor skips a block whose departure points can only reach bricks
 //     without (lysed) dye: its result there is exactly +0;
-//   - the reference resolve skips the voxels of a block that sees no predictor
-//     value within one voxel and no splat, and the box's those whose bracket is
-//     two zeros: the result there is exactly +0;
+//   - the reference resolve skips the bricks that see no predictor value within
+//     one voxel, no splat and no floor, and the box's those whose bracket is all
+//     zeros: the result there is exactly +0;
 //   - the zeros of a skipped voxel are stored only where the array's last
 //     contents (pold, cold: the flags before this step) may not be zero already;
 //   - the reference resolve reads the splat sums, the Casson stages the dye and
 //     the box's resolve the bracket only where the flags say there may be any.
 // So clear water costs flag reads, not the 5 to 9 words per voxel these stages
-// touch: reference Casson 54 -> 34 us and resolve 73 -> 58 us at 96x128x96 (dye
-// 192x256x192), the box's predictor and resolve 75 -> 47 and 44 -> 24 us at
-// 192x256x192.  (Casson of the box reads the dye everywhere: 76 us with the
+// touch: reference Casson 54 -> 34, predictor 30 -> 14 and resolve 73 -> 20 us at
+// 96x128x96 (dye 192x256x192), the box's predictor and resolve 75 -> 30 and 44
+// -> 15 us at 192x256x192, with the lists below.  (Casson of the box reads the dye everywhere: 76 us with the
 // flags, 78 without, all of it hidden behind the velocity's traffic.)  Flags are plain stores of 1 (a race between writers of the same
 // value is harmless); launch_dye_flags_begin clears them.
 // |centre velocity| per axis inside a step: the projection clamps the faces
 // to +-2 (fluid.ts:908) and the centre is their mean (with a margin)
 constexpr float kDyeSpeedBound = 2.0f * 1.0001f;
-constexpr int kDyeResolveZ = 4;  // voxels per thread along z in the sparse predictor and resolves (divides kDyeBrick)
 __device__ __forceinline__ void mark_brick(const Grid& gc, uint32_t* flags, int x, int y, int z) {
   flags[brick_of(gc, x, y, z)] = 1u;
 }
@@ -624,13 +623,12 @@ __device__ __forceinline__ int reach_voxels(float d, int n, float size) {
   const float r = ceilf(d * (float)n / size);
   return (r < (float)n ? (int)r : n) + 1;
 }
-__device__ __forceinline__ bool block_reaches_dye(const Grid& gc, const StepParams& P, const uint32_t* cbrick,
-                                                  float speed, int zlo, int zhi) {
-  const float d = speed * P.dt;
-  const int rx = reach_voxels(d, gc.nx, P.dsize[0]);
-  const int ry = reach_voxels(d, gc.ny, P.dsize[1]);
-  const int rz = reach_voxels(d, gc.nz, P.dsize[2]);
-  return block_any_brick(gc, cbrick, rx, ry, rz, zlo, zhi);
+struct Reach { int x, y, z; };
+__device__ __forceinline__ Reach dye_reach(const Grid& gc, const StepParams& P, const unsigned int* speedbits) {
+  // a margin of 1e-4 for the departure's rounding
+  const float d = (speedbits ? __uint_as_float(*speedbits) * 1.0001f : kDyeSpeedBound) * P.dt;
+  return Reach{reach_voxels(d, gc.nx, P.dsize[0]), reach_voxels(d, gc.ny, P.dsize[1]),
+               reach_voxels(d, gc.nz, P.dsize[2])};
 }
 
 // ---- CONC_PREDICT (advect.ts:28-72) -----------------------------------------------------------
@@ -688,11 +686,9 @@ __device__ __forceinline__ void predict_cell(const Grid& gc, const Grid& g, cons
   }
 }
 
-// ZP voxels per thread along z (grid z = nz / ZP): with the brick flags
-// (inside a step, ZP = kDyeResolveZ) one reach test serves ZP planes;
-// without them one voxel per thread.
-template <class VS, class DS, int ZP>
-__global__ void __launch_bounds__(256, ZP == 1 ? 8 : 4) k_conc_predict(Grid gc, Grid g, const StepParams* __restrict__ Pp, int ref,
+// One voxel per thread.
+template <class VS, class DS>
+__global__ void __launch_bounds__(256, 8) k_conc_predict(Grid gc, Grid g, const StepParams* __restrict__ Pp, int ref,
                                                       const typename Vec4Of<VS>::type* __restrict__ cen,
                                                       const typename Vec4Of<DS>::type* __restrict__ conc4,
                                                       const DS* __restrict__ dye, DS* __restrict__ pred,
@@ -701,30 +697,132 @@ __global__ void __launch_bounds__(256, ZP == 1 ? 8 : 4) k_conc_predict(Grid gc, 
                                                       const unsigned int* __restrict__ speedbits) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int z0 = blockIdx.z * ZP;
-  const int z1 = min(z0 + ZP, gc.nz);
+  const int z = blockIdx.z;
   const StepParams& P = *Pp;
-  // inside a step: a block whose departure points can only reach dye bricks
-  // holding nothing but +0 (reference mode: no lysed dye) writes the zeros
-  // the trace would give without tracing.  The centre velocity is bounded
-  // per axis by the projection's clamp to +-2 in reference mode, by the
-  // projection's own maximum (speedbits, a margin of 1e-4 for the
-  // departure's rounding) in the closed box.
+  // inside a step: a block that cannot reach dye (see k_dye_list) writes the
+  // zeros the trace would give without tracing
   if (cbrick) {
-    const float speed = speedbits ? __uint_as_float(*speedbits) * 1.0001f : kDyeSpeedBound;
-    if (!block_reaches_dye(gc, P, cbrick, speed, z0, z1 - 1)) {
-      if (x < gc.nx && y < gc.ny && brick_held(gc, pold, x, y, z0))
-        for (int z = z0; z < z1; ++z) {
-          const size_t i = gc.at(x, y, z);
-          stf(pred + i, 0.0f);
-          if (lim) { stf(lim + 2 * i, 0.0f); stf(lim + 2 * i + 1, 0.0f); }
-        }
+    const Reach r = dye_reach(gc, P, speedbits);
+    if (!block_any_brick(gc, cbrick, r.x, r.y, r.z, z, z)) {
+      if (x < gc.nx && y < gc.ny && brick_held(gc, pold, x, y, z)) {
+        const size_t i = gc.at(x, y, z);
+        stf(pred + i, 0.0f);
+        if (lim) { stf(lim + 2 * i, 0.0f); stf(lim + 2 * i + 1, 0.0f); }
+      }
       return;
     }
   }
   if (x >= gc.nx || y >= gc.ny) return;
+  predict_cell<VS, DS>(gc, g, P, ref, cen, conc4, dye, pred, lim, pbrick, x, y, z);
+}
+
+// The bricks of a large grid that a dye stage has to look at, as a list: a
+// block per 32 x 8 voxels of the whole grid spends about 2 us on finding out
+// that its water is clear, and the heavy stages' registers allow 3 or 4 blocks
+// per SM, so those blocks took 20 to 35 us of the predictor's 28 and the
+// reference resolve's 57 (dye 192x256x192).  One warp per brick here (one
+// thread per brick, 27 flags in a row, was slower: 271 against 256 us a
+// substep), then persistent blocks over the list, half a brick (256 voxels) at a time.
+//   kListPredict     a brick whose departure points can reach a flagged one:
+//                    the centre velocity is bounded per axis by the projection's
+//                    clamp to +-2 in reference mode, by the projection's own
+//                    maximum (speedbits) in the closed box
+//   kListResolveRef  the floor zone, a splat in the brick, or a predictor value
+//                    within one voxel (entry bit 31: none, its splat-free
+//                    voxels outside the floor zone are clear)
+//   kListResolveBox  a brick of the predictor's
+// Every other brick's result is +0, stored here where `old` says that the
+// array (PER values a voxel, and lim's two) may hold something else.
+enum DyeList { kListPredict, kListResolveRef, kListResolveBox };
+template <int MODE, class DS, int PER>
+__global__ void __launch_bounds__(256) k_dye_list(Grid gc, const StepParams* __restrict__ Pp,
+                                                  const uint32_t* __restrict__ flags,
+                                                  const uint32_t* __restrict__ sbrick,
+                                                  const uint32_t* __restrict__ old,
+                                                  const unsigned int* __restrict__ speedbits, DS* __restrict__ out,
+                                                  DS* __restrict__ lim, uint32_t* __restrict__ count,
+                                                  uint32_t* __restrict__ list) {
+  pdl_trigger();
+  __shared__ uint32_t marked, base;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (threadIdx.x == 0) marked = 0u;
+  __syncthreads();
+  const Grid bg = brick_grid(gc);
+  const int bx = blockIdx.x * 8 + warp, by = blockIdx.y, bz = blockIdx.z;
+  const bool in = bx < bg.nx;
+  const uint32_t b = (uint32_t)bg.at(bx, by, bz);
+  bool active = false, near = false;
+  if (in) {
+    if (MODE == kListResolveBox) {
+      active = flags[b] != 0u;
+    } else {
+      // bricks that the brick's voxels reach
+      int rx = 1, ry = 1, rz = 1;
+      if (MODE == kListPredict) {
+        const Reach r = dye_reach(gc, *Pp, speedbits);
+        rx = (r.x + kDyeBrick - 1) / kDyeBrick; ry = (r.y + kDyeBrick - 1) / kDyeBrick; rz = (r.z + kDyeBrick - 1) / kDyeBrick;
+      }
+      const int nx = 2 * rx + 1, ny = 2 * ry + 1, nz = 2 * rz + 1;
+      if (rx == 1 && ry == 1 && rz == 1) {
+        const int x = bx + lane % 3 - 1, y = by + (lane / 3) % 3 - 1, z = bz + lane / 9 - 1;
+        near = lane < 27 && x >= 0 && x < bg.nx && y >= 0 && y < bg.ny && z >= 0 && z < bg.nz && flags[bg.at(x, y, z)] != 0u;
+      } else {
+        for (int k = lane; k < nx * ny * nz && !near; k += 32) {
+          const int x = bx + k % nx - rx, y = by + (k / nx) % ny - ry, z = bz + k / (nx * ny) - rz;
+          near = x >= 0 && x < bg.nx && y >= 0 && y < bg.ny && z >= 0 && z < bg.nz && flags[bg.at(x, y, z)] != 0u;
+        }
+      }
+      near = __any_sync(0xffffffffu, near);
+      active = near;
+      if (MODE == kListResolveRef) active = near || by == 0 || sbrick[b] != 0u;
+    }
+    if (active && lane == 0) atomicOr(&marked, 1u << warp);
+  }
+  __syncthreads();
+  const uint32_t m = marked;
+  if (threadIdx.x == 0 && m) base = atomicAdd(count, (uint32_t)__popc(m));
+  __syncthreads();
+  if (!in) return;
+  if (active) {
+    if (lane == 0)
+      list[base + __popc(m & ((1u << warp) - 1u))] = b | (MODE == kListResolveRef && !near ? 0x80000000u : 0u);
+  } else if (old[b]) {
+    const int x = bx * kDyeBrick + (lane & 7);
+    for (int k = lane >> 3; k < kDyeBrick * kDyeBrick; k += 4) {
+      const int y = by * kDyeBrick + (k & 7), z = bz * kDyeBrick + (k >> 3);
+      if (x >= gc.nx || y >= gc.ny || z >= gc.nz) continue;
+      const size_t i = gc.at(x, y, z);
+#pragma unroll
+      for (int c = 0; c < PER; ++c) stf(out + PER * i + c, 0.0f);
+      if (lim) { stf(lim + 2 * i, 0.0f); stf(lim + 2 * i + 1, 0.0f); }
+    }
+  }
+}
+// f(x, y, z, entry) for the voxels of the listed bricks, one per thread
+template <class F>
+__device__ __forceinline__ void for_listed(const Grid& gc, const uint32_t* count, const uint32_t* list, F f) {
+  const Grid bg = brick_grid(gc);
+  const int tid = threadIdx.x;
+  const uint32_t n = 2u * *count;
 #pragma unroll 1
-  for (int z = z0; z < z1; ++z) predict_cell<VS, DS>(gc, g, P, ref, cen, conc4, dye, pred, lim, pbrick, x, y, z);
+  for (uint32_t u = blockIdx.x; u < n; u += gridDim.x) {
+    const uint32_t e = list[u >> 1], b = e & 0x7fffffffu;
+    const int x = (int)(b % bg.nx) * kDyeBrick + (tid & 7), y = (int)((b / bg.nx) % bg.ny) * kDyeBrick + ((tid >> 3) & 7);
+    const int z = (int)(b / ((uint32_t)bg.nx * bg.ny)) * kDyeBrick + (tid >> 6) + 4 * (int)(u & 1u);
+    if (x < gc.nx && y < gc.ny && z < gc.nz) f(x, y, z, e);
+  }
+}
+constexpr int kPredictBlocks = 4, kResolveRefBlocks = 3, kResolveBoxBlocks = 5;  // per SM
+template <class VS, class DS>
+__global__ void __launch_bounds__(256, kPredictBlocks) k_conc_predict_list(
+    Grid gc, Grid g, const StepParams* __restrict__ Pp, int ref, const typename Vec4Of<VS>::type* __restrict__ cen,
+    const typename Vec4Of<DS>::type* __restrict__ conc4, const DS* __restrict__ dye, DS* __restrict__ pred,
+    DS* __restrict__ lim, uint32_t* __restrict__ pbrick, const uint32_t* count, const uint32_t* list) {
+  pdl_wait();
+  const StepParams& P = *Pp;
+  for_listed(gc, count, list, [&](int x, int y, int z, uint32_t) {
+    predict_cell<VS, DS>(gc, g, P, ref, cen, conc4, dye, pred, lim, pbrick, x, y, z);
+  });
 }
 
 // ---- CONC_RESOLVE (advect.ts:81-298) ------------------------------------------------------------
@@ -864,61 +962,51 @@ __device__ __forceinline__ void resolve_ref_cell(const Grid& gc, const Grid& g, 
     mark_brick(gc, held_out, x, y, z);
 }
 
-// Each thread resolves kDyeResolveZ voxels along z: their splat sums are
-// loaded before the block's brick test, so in clear water (most of the dye
-// grid) the flag loads, the barrier and the splat loads overlap and one
-// test serves kDyeResolveZ planes; the voxels that need the full resolve
-// then run it one after another.
+// A voxel of the resolve: the boundary shell and clear water's early-out
+// (`clear`: every predictor tap +0, so oct0 = oct1 = 0 in resolve_ref_cell)
+// outside the floor zone hold zeros.
 template <class VS, class DS>
-__global__ void __launch_bounds__(256, 3) k_conc_resolve_ref(Grid gc, Grid g, const StepParams* __restrict__ Pp,
-                                                          const typename Vec4Of<VS>::type* __restrict__ cen,
-                                                          const typename Vec4Of<DS>::type* __restrict__ conc,
-                                                          const DS* __restrict__ pred,
-                                                          const uint32_t* __restrict__ splatI,
-                                                          const uint32_t* __restrict__ splatL,
-                                                          typename Vec4Of<DS>::type* __restrict__ out,
-                                                          const uint32_t* __restrict__ sbrick,
-                                                          const uint32_t* __restrict__ pbrick,
-                                                          const uint32_t* __restrict__ cold,
-                                                          uint32_t* __restrict__ cbrick_out,
-                                                          uint32_t* __restrict__ held_out) {
+__device__ __forceinline__ void resolve_ref_voxel(const Grid& gc, const Grid& g, const StepParams& P,
+                                                  const typename Vec4Of<VS>::type* __restrict__ cen,
+                                                  const typename Vec4Of<DS>::type* __restrict__ conc,
+                                                  const DS* __restrict__ pred, const uint32_t* __restrict__ splatI,
+                                                  const uint32_t* __restrict__ splatL,
+                                                  typename Vec4Of<DS>::type* __restrict__ out,
+                                                  uint32_t* __restrict__ cbrick_out, uint32_t* __restrict__ held_out,
+                                                  bool clear, int x, int y, int z) {
+  const size_t i = gc.at(x, y, z);
+  const bool shell = x == 0 || x >= gc.nx - 1 || y >= gc.ny - 1 || z == 0 || z >= gc.nz - 1;
+  if (shell || (clear && y > 7 && __ldg(splatI + i) == 0u && __ldg(splatL + i) == 0u))
+    st4(out + i, make_float4(0.f, 0.f, 0.f, 0.f));
+  else
+    resolve_ref_cell<VS, DS>(gc, g, P, cen, conc, pred, splatI, splatL, out, cbrick_out, held_out, x, y, z);
+}
+// every voxel, one per thread (the stage on its own)
+template <class VS, class DS>
+__global__ void __launch_bounds__(256, kResolveRefBlocks) k_conc_resolve_ref(
+    Grid gc, Grid g, const StepParams* __restrict__ Pp, const typename Vec4Of<VS>::type* __restrict__ cen,
+    const typename Vec4Of<DS>::type* __restrict__ conc, const DS* __restrict__ pred,
+    const uint32_t* __restrict__ splatI, const uint32_t* __restrict__ splatL,
+    typename Vec4Of<DS>::type* __restrict__ out, uint32_t* __restrict__ cbrick_out, uint32_t* __restrict__ held_out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int z0 = blockIdx.z * kDyeResolveZ;
-  const bool inside = x < gc.nx && y < gc.ny;
-  const bool splats = inside && brick_held(gc, sbrick, x, y, z0);
-  const bool held = inside && brick_held(gc, cold, x, y, z0);
-  uint32_t rI[kDyeResolveZ], rL[kDyeResolveZ];
-#pragma unroll
-  for (int k = 0; k < kDyeResolveZ; ++k) {
-    const bool ok = splats && z0 + k < gc.nz;
-    const size_t i = ok ? gc.at(x, y, z0 + k) : 0;
-    rI[k] = ok ? __ldg(splatI + i) : 0u;
-    rL[k] = ok ? __ldg(splatL + i) : 0u;
-  }
-  // inside a step: no predictor value within one voxel of the block
-  const bool clear = pbrick && !block_any_brick(gc, pbrick, 1, 1, 1, z0, z0 + kDyeResolveZ - 1);
-  if (!inside) return;
-  const bool shellXY = x == 0 || x >= gc.nx - 1 || y >= gc.ny - 1;
-  const bool inFloorZone = y <= 7;
-  unsigned need = 0u;
-#pragma unroll
-  for (int k = 0; k < kDyeResolveZ; ++k) {
-    const int z = z0 + k;
-    if (z >= gc.nz) break;
-    // the boundary shell, and clear water's early-out (every predictor tap
-    // +0, so oct0 = oct1 = 0 below) outside the floor zone
-    if (!(shellXY || z == 0 || z >= gc.nz - 1 || (clear && !inFloorZone && rI[k] == 0u && rL[k] == 0u)))
-      need |= 1u << k;
-    else if (held)
-      st4(out + gc.at(x, y, z), make_float4(0.f, 0.f, 0.f, 0.f));
-  }
+  if (x >= gc.nx || y >= gc.ny) return;
+  resolve_ref_voxel<VS, DS>(gc, g, *Pp, cen, conc, pred, splatI, splatL, out, cbrick_out, held_out, false, x, y,
+                            blockIdx.z);
+}
+// the listed bricks' (inside a step)
+template <class VS, class DS>
+__global__ void __launch_bounds__(256, kResolveRefBlocks) k_conc_resolve_ref_list(
+    Grid gc, Grid g, const StepParams* __restrict__ Pp, const typename Vec4Of<VS>::type* __restrict__ cen,
+    const typename Vec4Of<DS>::type* __restrict__ conc, const DS* __restrict__ pred,
+    const uint32_t* __restrict__ splatI, const uint32_t* __restrict__ splatL,
+    typename Vec4Of<DS>::type* __restrict__ out, uint32_t* __restrict__ cbrick_out, uint32_t* __restrict__ held_out,
+    const uint32_t* count, const uint32_t* list) {
+  pdl_wait();
   const StepParams& P = *Pp;
-  while (need) {
-    const int k = __ffs(need) - 1;
-    need &= need - 1u;
-    resolve_ref_cell<VS, DS>(gc, g, P, cen, conc, pred, splatI, splatL, out, cbrick_out, held_out, x, y, z0 + k);
-  }
+  for_listed(gc, count, list, [&](int x, int y, int z, uint32_t e) {
+    resolve_ref_voxel<VS, DS>(gc, g, P, cen, conc, pred, splatI, splatL, out, cbrick_out, held_out, e >> 31, x, y, z);
+  });
 }
 
 // Closed box: MacCormack correction of the single dye, 8-tap min/max limiter.
@@ -988,11 +1076,11 @@ __device__ __forceinline__ void resolve_lim_cell(const Grid& gc, const Grid& g, 
   stf(out + i, r);
   if (cbrick_out && __float_as_uint(r) != 0u) mark_brick(gc, cbrick_out, x, y, z);
 }
-// ZP voxels per thread along z.  pbrick (inside a step): where the
-// predictor left its arrays at +0, the bracket is not read, and the zero is
-// stored only where cold says that `out` may hold something else.
-template <class VS, class DS, int ZP>
-__global__ void __launch_bounds__(256, ZP == 1 ? 8 : 5) k_dye_resolve_lim(Grid gc, Grid g, const StepParams* __restrict__ Pp,
+// One voxel per thread.  pbrick (inside a step): where the predictor left its
+// arrays at +0, the bracket is not read, and the zero is stored only where
+// cold says that `out` may hold something else.
+template <class VS, class DS>
+__global__ void __launch_bounds__(256, 8) k_dye_resolve_lim(Grid gc, Grid g, const StepParams* __restrict__ Pp,
                                                          const typename Vec4Of<VS>::type* __restrict__ cen,
                                                          const DS* __restrict__ dye, const DS* __restrict__ pred,
                                                          const DS* __restrict__ lim, DS* __restrict__ out,
@@ -1001,15 +1089,25 @@ __global__ void __launch_bounds__(256, ZP == 1 ? 8 : 5) k_dye_resolve_lim(Grid g
                                                          uint32_t* __restrict__ cbrick_out) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int z0 = blockIdx.z * ZP, z1 = min(z0 + ZP, gc.nz);
+  const int z = blockIdx.z;
   if (x >= gc.nx || y >= gc.ny) return;
-  if (!brick_held(gc, pbrick, x, y, z0)) {
-    if (brick_held(gc, cold, x, y, z0))
-      for (int z = z0; z < z1; ++z) stf(out + gc.at(x, y, z), 0.0f);
+  if (!brick_held(gc, pbrick, x, y, z)) {
+    if (brick_held(gc, cold, x, y, z)) stf(out + gc.at(x, y, z), 0.0f);
     return;
   }
-#pragma unroll 1
-  for (int z = z0; z < z1; ++z) resolve_lim_cell<VS, DS>(gc, g, *Pp, cen, dye, pred, lim, out, cbrick_out, x, y, z);
+  resolve_lim_cell<VS, DS>(gc, g, *Pp, cen, dye, pred, lim, out, cbrick_out, x, y, z);
+}
+// the listed bricks' (inside a step)
+template <class VS, class DS>
+__global__ void __launch_bounds__(256, kResolveBoxBlocks) k_dye_resolve_lim_list(
+    Grid gc, Grid g, const StepParams* __restrict__ Pp, const typename Vec4Of<VS>::type* __restrict__ cen,
+    const DS* __restrict__ dye, const DS* __restrict__ pred, const DS* __restrict__ lim, DS* __restrict__ out,
+    uint32_t* __restrict__ cbrick_out, const uint32_t* count, const uint32_t* list) {
+  pdl_wait();
+  const StepParams& P = *Pp;
+  for_listed(gc, count, list, [&](int x, int y, int z, uint32_t) {
+    resolve_lim_cell<VS, DS>(gc, g, P, cen, dye, pred, lim, out, cbrick_out, x, y, z);
+  });
 }
 
 // ---- host launchers ------------------------------------------------------------------------------
@@ -1116,12 +1214,15 @@ void launch_dye_bricks_unknown(const DevState& s, cudaStream_t st) {
 }
 size_t dye_brick_count(const Grid& gc) { return brick_grid(gc).n(); }
 
-// Old flags kept (pold, cold), the flags of what this step writes cleared.
+// Old flags kept (pold, cold), the flags of what this step writes and the
+// lists' counts cleared.
 __global__ void __launch_bounds__(256) k_dye_flags_begin(size_t nb, uint32_t* __restrict__ pbrick,
                                                          uint32_t* __restrict__ pold, uint32_t* __restrict__ held_out,
                                                          uint32_t* __restrict__ cold,
-                                                         uint32_t* __restrict__ cbrick_out) {
+                                                         uint32_t* __restrict__ cbrick_out,
+                                                         uint32_t* __restrict__ counts) {
   const size_t b = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+  if (b < 2) counts[b] = 0u;
   if (b >= nb) return;
   pold[b] = pbrick[b];
   pbrick[b] = 0u;
@@ -1132,16 +1233,22 @@ __global__ void __launch_bounds__(256) k_dye_flags_begin(size_t nb, uint32_t* __
 void launch_dye_flags_begin(const DevState& s, cudaStream_t st) {
   const size_t nb = brick_grid(s.gc).n();
   k_dye_flags_begin<<<(unsigned)((nb + 255) / 256), 256, 0, st>>>(nb, s.pbrick, s.pold, held_flags_of(s, s.conc2),
-                                                                 s.cold, brick_flags_of(s, s.conc2));
+                                                                 s.cold, brick_flags_of(s, s.conc2), s.dye_list);
 }
 
-// The closed box's sparse predictor and resolve take kDyeResolveZ voxels per
-// thread where that still gives 8 blocks per SM (192x256x192: predictor 75 ->
-// 47 us, resolve 44 -> 24), else one (48x64x48: 9.5 and 7.5 us, 11.8 and 10.0
-// with four; 96x128x96: resolve 10.4, 12.5 with four).
-static bool sparse_planes(const DevState& s) {
-  const dim3 gr = cell_grid(s.gc);
-  return (size_t)gr.x * gr.y * gr.z >= (size_t)kDyeResolveZ * 8 * s.num_sms;
+// Lists from a million voxels: at 96x128x96 (1.2 million) the predictor takes
+// 14.9 us with the list and 18.2 without, at 72x104x56 (419 thousand) 11.1 and
+// 12.5 but the resolve 9.6 and 8.1 (steps 252 and 250 us): there the list's
+// launch costs what it saves.  The reference resolve, whose stage is heavier,
+// is always listed.
+static bool dye_listed(const DevState& s) { return s.gc.n() >= 1000000u; }
+template <int MODE, class DS, int PER>
+static void launch_dye_list(const DevState& s, const uint32_t* flags, const uint32_t* old, const unsigned int* speed,
+                            void* out, void* lim, cudaStream_t st) {
+  const Grid b = brick_grid(s.gc);
+  k_dye_list<MODE, DS, PER><<<dim3((b.nx + 7) / 8, b.ny, b.nz), 256, 0, st>>>(
+      s.gc, s.params, flags, s.sbrick, old, speed, (DS*)out, (DS*)lim, s.dye_list + (MODE != kListPredict),
+      s.dye_list + 2);
 }
 
 void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket, bool sparse) {
@@ -1149,32 +1256,39 @@ void launch_conc_predict(const DevState& s, cudaStream_t st, bool bracket, bool 
   // outside a step the predictor's arrays (the tape's share the bracket)
   // may then hold anything
   if (!sparse && s.pbrick) cudaMemsetAsync(s.pbrick, 1, brick_grid(s.gc).n() * sizeof(uint32_t), st);
+  void* lim = bracket && !s.ref ? s.lim : nullptr;
+  // the closed box's bound on the centre velocity comes from the projection
+  const unsigned int* speed = cb && !s.ref ? s.redu + REDU_SPEED : nullptr;
   DOB_VEL_DISPATCH(s.prec, {
-    auto run = [&](auto* k, int zp) {
-      dim3 gr = cell_grid(s.gc);
-      gr.z = (s.gc.nz + zp - 1) / zp;
-      // the closed box's bound on the centre velocity comes from the projection
-      k<<<gr, cell_block(), 0, st>>>(s.gc, s.g, s.params, s.ref, (const typename Vec4Of<VS>::type*)s.cen,
-                                     (const typename Vec4Of<DS>::type*)s.conc, (const DS*)s.conc, (DS*)s.pred,
-                                     bracket && !s.ref ? (DS*)s.lim : nullptr, cb, sparse ? s.pbrick : nullptr, s.pold,
-                                     cb && !s.ref ? s.redu + REDU_SPEED : nullptr);
-    };
-    if (cb && (s.ref || sparse_planes(s))) run(k_conc_predict<VS, DS, kDyeResolveZ>, kDyeResolveZ);
-    else run(k_conc_predict<VS, DS, 1>, 1);
+    using V4 = typename Vec4Of<VS>::type;
+    using D4 = typename Vec4Of<DS>::type;
+    if (cb && dye_listed(s)) {
+      launch_dye_list<kListPredict, DS, 1>(s, cb, s.pold, speed, s.pred, lim, st);
+      launch_pdl(k_conc_predict_list<VS, DS>, dim3(s.num_sms * kPredictBlocks), dim3(256), 0, st, s.gc, s.g, s.params,
+                 s.ref, (const V4*)s.cen, (const D4*)s.conc, (const DS*)s.conc, (DS*)s.pred, (DS*)lim, s.pbrick,
+                 (const uint32_t*)s.dye_list, (const uint32_t*)(s.dye_list + 2));
+    } else {
+      k_conc_predict<VS, DS><<<cell_grid(s.gc), cell_block(), 0, st>>>(
+          s.gc, s.g, s.params, s.ref, (const V4*)s.cen, (const D4*)s.conc, (const DS*)s.conc, (DS*)s.pred, (DS*)lim,
+          cb, sparse ? s.pbrick : nullptr, s.pold, speed);
+    }
   });
 }
 
 void launch_dye_resolve_lim(const DevState& s, cudaStream_t st, bool sparse) {
+  uint32_t* cb = brick_flags_of(s, s.conc2);
   DOB_VEL_DISPATCH(s.prec, {
-    auto run = [&](auto* k, int zp) {
-      dim3 gr = cell_grid(s.gc);
-      gr.z = (s.gc.nz + zp - 1) / zp;
-      k<<<gr, cell_block(), 0, st>>>(s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const DS*)s.conc,
-                                     (const DS*)s.pred, (const DS*)s.lim, (DS*)s.conc2, sparse ? s.pbrick : nullptr,
-                                     sparse ? s.cold : nullptr, brick_flags_of(s, s.conc2));
-    };
-    if (sparse && sparse_planes(s)) run(k_dye_resolve_lim<VS, DS, kDyeResolveZ>, kDyeResolveZ);
-    else run(k_dye_resolve_lim<VS, DS, 1>, 1);
+    using V4 = typename Vec4Of<VS>::type;
+    if (sparse && dye_listed(s)) {
+      launch_dye_list<kListResolveBox, DS, 1>(s, s.pbrick, s.cold, nullptr, s.conc2, nullptr, st);
+      launch_pdl(k_dye_resolve_lim_list<VS, DS>, dim3(s.num_sms * kResolveBoxBlocks), dim3(256), 0, st, s.gc, s.g,
+                 s.params, (const V4*)s.cen, (const DS*)s.conc, (const DS*)s.pred, (const DS*)s.lim, (DS*)s.conc2, cb,
+                 (const uint32_t*)(s.dye_list + 1), (const uint32_t*)(s.dye_list + 2));
+    } else {
+      k_dye_resolve_lim<VS, DS><<<cell_grid(s.gc), cell_block(), 0, st>>>(
+          s.gc, s.g, s.params, (const V4*)s.cen, (const DS*)s.conc, (const DS*)s.pred, (const DS*)s.lim, (DS*)s.conc2,
+          sparse ? s.pbrick : nullptr, sparse ? s.cold : nullptr, cb);
+    }
   });
 }
 
@@ -1188,17 +1302,21 @@ void launch_conc_resolve(const DevState& s, cudaStream_t st, bool sparse) {
       if (f) cudaMemsetAsync(f, s.ref ? 0 : 1, nb, st);
   }
   DOB_VEL_DISPATCH(s.prec, {
-    if (s.ref) {
-      dim3 gr = cell_grid(s.gc);
-      gr.z = (s.gc.nz + kDyeResolveZ - 1) / kDyeResolveZ;
-      k_conc_resolve_ref<VS, DS><<<gr, cell_block(), 0, st>>>(
-          s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const typename Vec4Of<DS>::type*)s.conc,
-          (const DS*)s.pred, s.splatI, s.splatL, (typename Vec4Of<DS>::type*)s.conc2, s.sbrick,
-          sparse ? s.pbrick : nullptr, sparse ? s.cold : nullptr, cb, hb);
+    using V4 = typename Vec4Of<VS>::type;
+    using D4 = typename Vec4Of<DS>::type;
+    if (s.ref && sparse) {
+      launch_dye_list<kListResolveRef, DS, 4>(s, s.pbrick, s.cold, nullptr, s.conc2, nullptr, st);
+      launch_pdl(k_conc_resolve_ref_list<VS, DS>, dim3(s.num_sms * kResolveRefBlocks), dim3(256), 0, st, s.gc, s.g,
+                 s.params, (const V4*)s.cen, (const D4*)s.conc, (const DS*)s.pred, (const uint32_t*)s.splatI,
+                 (const uint32_t*)s.splatL, (D4*)s.conc2, cb, hb, (const uint32_t*)(s.dye_list + 1),
+                 (const uint32_t*)(s.dye_list + 2));
+    } else if (s.ref) {
+      k_conc_resolve_ref<VS, DS><<<cell_grid(s.gc), cell_block(), 0, st>>>(
+          s.gc, s.g, s.params, (const V4*)s.cen, (const D4*)s.conc, (const DS*)s.pred, s.splatI, s.splatL,
+          (D4*)s.conc2, cb, hb);
     } else {
       k_dye_resolve_box<VS, DS><<<cell_grid(s.gc), cell_block(), 0, st>>>(
-          s.gc, s.g, s.params, (const typename Vec4Of<VS>::type*)s.cen, (const DS*)s.conc, (const DS*)s.pred,
-          (DS*)s.conc2);
+          s.gc, s.g, s.params, (const V4*)s.cen, (const DS*)s.conc, (const DS*)s.pred, (DS*)s.conc2);
     }
   });
 }

@@ -3,8 +3,8 @@ holds already is not stored again, and dye, bracket and splats are read only
 where there may be any) against the same steps with every flag set: a field
 written from outside marks every brick.  The same bits are required: a
 skipped value is a +0 either way, and splat sums are integers.  Grids with
-remainders in the bricks and blocks, and large enough for several voxels per
-thread; between steps the dye is replaced, single stages run and a snapshot is
+remainders in the bricks, below and above a million voxels (from where the
+stages work on a list of bricks); between steps the dye is replaced, single stages run and a snapshot is
 restored, so flags and arrays are seen in every order."""
 import numpy as np
 import pytest
@@ -37,7 +37,7 @@ def _run(sims, abi, ref, act, steps):
     np.testing.assert_array_equal(a.get_parcels(), b.get_parcels())
 
 
-@pytest.mark.parametrize("dims", [(16, 16, 16), (40, 56, 24), (72, 104, 56), (128, 128, 96)])
+@pytest.mark.parametrize("dims", [(16, 16, 16), (40, 56, 24), (72, 104, 56), (136, 92, 104)])
 @pytest.mark.parametrize("mixed", [False, True])
 def test_closed_box(dims, mixed):
     from dropfluid import DropFluid, abi
