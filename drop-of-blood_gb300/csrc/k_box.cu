@@ -7,7 +7,7 @@
 // rows.
 //
 // Each kernel computes exactly the expressions of its general counterpart in
-// k_fluid.cu (k_casson's closed-box branch, k_mac_rhs, k_project followed by
+// k_fluid.cu (k_casson, k_mac_rhs, k_project followed by
 // k_mac_to_center), in the same order, so the results are the same bits;
 // the step graph of the closed box uses these, the stage-level interface the
 // general kernels.
@@ -200,8 +200,6 @@ __global__ void __launch_bounds__(256, DOB_PROJECT_MIN_BLOCKS) k_project_center_
   if (speedbits) block_max_u32(smax, speedbits);
 }
 
-template <int ZC>
-inline dim3 col_grid(const Grid& g) { return dim3((g.nx + 31) / 32, (g.ny + 7) / 8, (g.nz + ZC - 1) / ZC); }
 constexpr int kCassonZ = 8, kRhsZ = 8, kProjectZ = 4;  // planes per thread (measured at 192x256x192)
 
 }  // namespace
@@ -212,20 +210,27 @@ bool box_casson_applies(const DevState& s) {
 
 void launch_casson_box(const DevState& s, cudaStream_t st) {
   DOB_VEL_DISPATCH(s.prec, {
-    k_casson_box<VS, DS, kCassonZ><<<col_grid<kCassonZ>(s.g), dim3(32, 8), 0, st>>>(
-        s.g, s.params, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w, (const DS*)s.conc, (VS*)s.u2, (VS*)s.v2,
-        (VS*)s.w2);
+    auto run = [&](auto* k, int zc) {
+      k<<<col_grid(s.g, zc), dim3(32, 8), 0, st>>>(s.g, s.params, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w,
+                                                   (const DS*)s.conc, (VS*)s.u2, (VS*)s.v2, (VS*)s.w2);
+    };
+    if (long_columns(s, kCassonZ)) run(k_casson_box<VS, DS, kCassonZ>, kCassonZ);
+    else run(k_casson_box<VS, DS, kShortZ>, kShortZ);
   });
 }
 
 void launch_mac_rhs_box(const DevState& s, cudaStream_t st, double* sumsq) {
   DOB_VEL_DISPATCH(s.prec, {
-    if (s.g.nz % kRhsZ == 0)
-      k_rhs_box<VS, kRhsZ, true><<<col_grid<kRhsZ>(s.g), dim3(32, 8), 0, st>>>(s.g, (const VS*)s.u, (const VS*)s.v,
-                                                                             (const VS*)s.w, s.rhs);
-    else
-      k_rhs_box<VS, kRhsZ, false><<<col_grid<kRhsZ>(s.g), dim3(32, 8), 0, st>>>(s.g, (const VS*)s.u, (const VS*)s.v,
-                                                                              (const VS*)s.w, s.rhs);
+    auto run = [&](auto* k, int zc) {
+      k<<<col_grid(s.g, zc), dim3(32, 8), 0, st>>>(s.g, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w, s.rhs);
+    };
+    if (!long_columns(s, kRhsZ)) {
+      run(k_rhs_box<VS, kShortZ, true>, kShortZ);
+    } else if (s.g.nz % kRhsZ == 0) {
+      run(k_rhs_box<VS, kRhsZ, true>, kRhsZ);
+    } else {
+      run(k_rhs_box<VS, kRhsZ, false>, kRhsZ);
+    }
   });
   launch_sum(s.rhs, s.g.n(), s.part + PART_RHS * kSumBlocks, s.num_sms, st);
   launch_sub_mean(s.rhs, s.g.n(), s.part + PART_RHS * kSumBlocks, s.num_sms, st, sumsq);
@@ -234,14 +239,18 @@ void launch_mac_rhs_box(const DevState& s, cudaStream_t st, double* sumsq) {
 void launch_project_center_box(const DevState& s, cudaStream_t st, float scale, unsigned int* maxbits,
                                unsigned int* speedbits) {
   DOB_VEL_DISPATCH(s.prec, {
-    if (s.g.nz % kProjectZ == 0)
-      k_project_center_box<VS, kProjectZ, true><<<col_grid<kProjectZ>(s.g), dim3(32, 8), 0, st>>>(
-          s.g, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w, s.p, s.plo, (VS*)s.u2, (VS*)s.v2, (VS*)s.w2,
-          (typename Vec4Of<VS>::type*)s.cen, scale, maxbits, speedbits);
-    else
-      k_project_center_box<VS, kProjectZ, false><<<col_grid<kProjectZ>(s.g), dim3(32, 8), 0, st>>>(
-          s.g, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w, s.p, s.plo, (VS*)s.u2, (VS*)s.v2, (VS*)s.w2,
-          (typename Vec4Of<VS>::type*)s.cen, scale, maxbits, speedbits);
+    auto run = [&](auto* k, int zc) {
+      k<<<col_grid(s.g, zc), dim3(32, 8), 0, st>>>(s.g, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w, s.p, s.plo,
+                                                   (VS*)s.u2, (VS*)s.v2, (VS*)s.w2,
+                                                   (typename Vec4Of<VS>::type*)s.cen, scale, maxbits, speedbits);
+    };
+    if (!long_columns(s, kProjectZ)) {
+      run(k_project_center_box<VS, kShortZ, true>, kShortZ);
+    } else if (s.g.nz % kProjectZ == 0) {
+      run(k_project_center_box<VS, kProjectZ, true>, kProjectZ);
+    } else {
+      run(k_project_center_box<VS, kProjectZ, false>, kProjectZ);
+    }
   });
 }
 

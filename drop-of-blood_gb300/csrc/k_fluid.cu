@@ -5,6 +5,7 @@
 // Each kernel is one HBM-bound pass over the grid (one thread per cell,
 // x-fastest warps so every field access is a coalesced row segment; the
 // trilinear gathers of the centre field are 16 B AoS loads).
+#include "dob_column.cuh"
 #include "dob_kernels.cuh"
 
 namespace dob {
@@ -322,7 +323,7 @@ __global__ void __launch_bounds__(256) k_curl(Grid g, const typename Vec4Of<VS>:
 //   - the reference resolve reads the splat sums, the Casson stages the dye and
 //     the box's resolve the bracket only where the flags say there may be any.
 // So clear water costs flag reads, not the 5 to 9 words per voxel these stages
-// touch: reference Casson 54 -> 34, predictor 30 -> 14 and resolve 73 -> 20 us at
+// touch: reference Casson 54 -> 34 (30 on columns), predictor 30 -> 14 and resolve 73 -> 20 us at
 // 96x128x96 (dye 192x256x192), the box's predictor and resolve 75 -> 30 and 44
 // -> 15 us at 192x256x192, with the lists below.  (Casson of the box reads the dye everywhere: 76 us with the
 // flags, 78 without, all of it hidden behind the velocity's traffic.)  Flags are plain stores of 1 (a race between writers of the same
@@ -393,39 +394,50 @@ __device__ __forceinline__ dob_v3 sample_conc_rg(const Grid& gc, const typename 
   return v3(r.x, r.y, 0.0f);
 }
 
-template <class VS, class DS>
-__global__ void __launch_bounds__(256) k_casson(Grid g, Grid gc, const StepParams* __restrict__ Pp, int ref, int flags,
-                                                const VS* __restrict__ u, const VS* __restrict__ v,
-                                                const VS* __restrict__ w,
-                                                const typename Vec4Of<VS>::type* __restrict__ curl,
-                                                const typename Vec4Of<DS>::type* __restrict__ conc4,
-                                                const DS* __restrict__ dye, const uint32_t* __restrict__ held,
-                                                VS* __restrict__ uo, VS* __restrict__ vo, VS* __restrict__ wo) {
-  // held (reference mode inside a step): the dye's flags.  The cell's two
-  // samples, at its centre and on its upper y face, tap dye voxels r x - 1 to
-  // r (x + 1) per axis (r dye cells per cell); one more for the rounding of
-  // the texel and 1/1000 of the axis, by which the face sample is clamped into
-  // the domain.  Over clear water both are +0 and not formed.
+// Reference mode, on z-columns (dob_column.cuh): the same expressions in the
+// same order as one thread per cell formed them with 18 clamped loads around
+// it (630 instructions a warp; FIGURES).
+// held (inside a step): the dye's flags.  The cell's two samples, at its
+// centre and on its upper y face, tap dye voxels r x - 1 to r (x + 1) per axis
+// (r dye cells per cell); one more for the rounding of the texel and 1/1000 of
+// the axis, by which the face sample is clamped into the domain.  Over clear
+// water both are +0 and not formed.
+template <class VS, class DS, int ZC>
+__global__ void __launch_bounds__(256, 4) k_casson_ref(Grid g, Grid gc, const StepParams* __restrict__ Pp, int flags,
+                                                    const VS* __restrict__ u, const VS* __restrict__ v,
+                                                    const VS* __restrict__ w,
+                                                    const typename Vec4Of<VS>::type* __restrict__ curl,
+                                                    const typename Vec4Of<DS>::type* __restrict__ conc4,
+                                                    const uint32_t* __restrict__ held, VS* __restrict__ uo,
+                                                    VS* __restrict__ vo, VS* __restrict__ wo) {
+  const Col c = column<ZC>(g);
+  if (c.z0 >= g.nz) return;  // uniform over the block
   bool dyed = true;
   if (held) {
     const int r = gc.nx / g.nx;
-    const int x0 = (int)(blockIdx.x * blockDim.x) * r, y0 = (int)(blockIdx.y * blockDim.y) * r, z0 = (int)blockIdx.z * r;
+    const int x0 = (int)(blockIdx.x * blockDim.x) * r, y0 = (int)(blockIdx.y * blockDim.y) * r;
     const int mx = 2 + gc.nx / 1000, my = 2 + gc.ny / 1000, mz = 2 + gc.nz / 1000;
-    dyed = any_brick(gc, held, x0 - mx, x0 + (int)blockDim.x * r + mx, y0 - my, y0 + (int)blockDim.y * r + my, z0 - mz,
-                     z0 + r + mz);
+    dyed = any_brick(gc, held, x0 - mx, x0 + (int)blockDim.x * r + mx, y0 - my, y0 + (int)blockDim.y * r + my,
+                     c.z0 * r - mz, c.zend * r + mz);
   }
-  CELL_INDEX
   const StepParams& P = *Pp;
   const Recip3 dims = grid_recip(g);
   const float dtv = P.dt;
-  dob_v3 mac = v3(ldf(u + i), ldf(v + i), ldf(w + i));
-  const dob_v3 mXp = ldmac(g, u, v, w, x + 1, y, z), mXn = ldmac(g, u, v, w, x - 1, y, z);
-  const dob_v3 mYp = ldmac(g, u, v, w, x, y + 1, z), mYn = ldmac(g, u, v, w, x, y - 1, z);
-  const dob_v3 mZp = ldmac(g, u, v, w, x, y, z + 1), mZn = ldmac(g, u, v, w, x, y, z - 1);
-  const dob_v3 uvwCell = (v3((float)x, (float)y, (float)z) + v3(0.5f, 0.5f, 0.5f)) / dims;
-  const dob_v3 du = mXp - mXn, dv = mYp - mYn, dw = mZp - mZn;
-  const dob_v3 lapMac = (mXp + mXn + mYp + mYn + mZp + mZn) - 6.0f * mac;
-  if (ref) {
+  const int x = c.x, y = c.y;
+  const int dym = y > 0 ? -(int)c.sy : 0, dyp = y < g.ny - 1 ? (int)c.sy : 0;
+  uint32_t i = c.i;
+  dob_v3 mZn = ld3(u, v, w, c.z0 > 0 ? i - c.sz : i);
+  dob_v3 own = ld3(u, v, w, i);
+#pragma unroll 1
+  for (int z = c.z0; z < c.zend; ++z) {
+    dob_v3 mac = own;
+    const dob_v3 mZp = ld3(u, v, w, z < g.nz - 1 ? i + c.sz : i);
+    const dob_v3 mXn = v3(x_minus(c, mac.x, u, i), x_minus(c, mac.y, v, i), x_minus(c, mac.z, w, i));
+    const dob_v3 mXp = v3(x_plus(c, g, mac.x, u, i), x_plus(c, g, mac.y, v, i), x_plus(c, g, mac.z, w, i));
+    const dob_v3 mYp = ld3(u, v, w, i + dyp), mYn = ld3(u, v, w, i + dym);
+    const dob_v3 uvwCell = (v3((float)x, (float)y, (float)z) + v3(0.5f, 0.5f, 0.5f)) / dims;
+    const dob_v3 du = mXp - mXn, dv = mYp - mYn, dw = mZp - mZn;
+    const dob_v3 lapMac = (mXp + mXn + mYp + mYn + mZp + mZn) - 6.0f * mac;
     const dob_v3 concCell = dyed ? sample_conc_rg<DS>(gc, conc4, uvwCell) : v3(0.0f, 0.0f, 0.0f);
     const float cRbc = dob_clampf(concCell.x, 0.0f, 1.5f);
     const float cassonScale = P.U[58];
@@ -478,22 +490,45 @@ __global__ void __launch_bounds__(256) k_casson(Grid g, Grid gc, const StepParam
       }
     }
     mac = clamp3(mac, -1.8f, 1.8f);
-  } else {
-    // Closed box: nu = (sqrt(mu_p) + sqrt(tau_y c^2 / (gdot + 0.4)))^2, explicit
-    // u += min(nu dt / dx^2, 1/8) lap u.
-    const float cval = gc.nx == g.nx ? ldf(dye + i) : lerp8(make_taps(gc, uvwCell.x, uvwCell.y, uvwCell.z), dye);
-    const float c = dob_clampf(cval, 0.0f, 1.5f);
-    const float dxv = P.dx;
-    const float gdot = dob_sqrt(dot3(du, du) + dot3(dv, dv) + dot3(dw, dw)) / (2.0f * dxv);
-    const float sqrtMu = dob_sqrt(P.mu_p);
-    const float sqrtYield = dob_sqrt(P.tau_y * c * c / (gdot + 0.4f));
-    const float nu = (sqrtMu + sqrtYield) * (sqrtMu + sqrtYield);
-    const float alpha = dob_minf(nu * dtv / (dxv * dxv), 0.125f);
-    mac = mac + alpha * lapMac;
+    if (x >= g.nx - 1) mac.x = 0.0f;
+    if (z >= g.nz - 1) mac.z = 0.0f;
+    if (c.valid) { stf(uo + i, mac.x); stf(vo + i, mac.y); stf(wo + i, mac.z); }
+    mZn = own;
+    own = mZp;
+    i += c.sz;
   }
+}
+
+// Closed box, any dye grid: nu = (sqrt(mu_p) + sqrt(tau_y c^2 / (gdot + 0.4)))^2,
+// explicit u += min(nu dt / dx^2, 1/8) lap u.
+template <class VS, class DS>
+__global__ void __launch_bounds__(256) k_casson(Grid g, Grid gc, const StepParams* __restrict__ Pp,
+                                                const VS* __restrict__ u, const VS* __restrict__ v,
+                                                const VS* __restrict__ w, const DS* __restrict__ dye,
+                                                VS* __restrict__ uo, VS* __restrict__ vo, VS* __restrict__ wo) {
+  CELL_INDEX
+  const StepParams& P = *Pp;
+  const Recip3 dims = grid_recip(g);
+  const float dtv = P.dt;
+  dob_v3 mac = v3(ldf(u + i), ldf(v + i), ldf(w + i));
+  const dob_v3 mXp = ldmac(g, u, v, w, x + 1, y, z), mXn = ldmac(g, u, v, w, x - 1, y, z);
+  const dob_v3 mYp = ldmac(g, u, v, w, x, y + 1, z), mYn = ldmac(g, u, v, w, x, y - 1, z);
+  const dob_v3 mZp = ldmac(g, u, v, w, x, y, z + 1), mZn = ldmac(g, u, v, w, x, y, z - 1);
+  const dob_v3 uvwCell = (v3((float)x, (float)y, (float)z) + v3(0.5f, 0.5f, 0.5f)) / dims;
+  const dob_v3 du = mXp - mXn, dv = mYp - mYn, dw = mZp - mZn;
+  const dob_v3 lapMac = (mXp + mXn + mYp + mYn + mZp + mZn) - 6.0f * mac;
+  const float cval = gc.nx == g.nx ? ldf(dye + i) : lerp8(make_taps(gc, uvwCell.x, uvwCell.y, uvwCell.z), dye);
+  const float c = dob_clampf(cval, 0.0f, 1.5f);
+  const float dxv = P.dx;
+  const float gdot = dob_sqrt(dot3(du, du) + dot3(dv, dv) + dot3(dw, dw)) / (2.0f * dxv);
+  const float sqrtMu = dob_sqrt(P.mu_p);
+  const float sqrtYield = dob_sqrt(P.tau_y * c * c / (gdot + 0.4f));
+  const float nu = (sqrtMu + sqrtYield) * (sqrtMu + sqrtYield);
+  const float alpha = dob_minf(nu * dtv / (dxv * dxv), 0.125f);
+  mac = mac + alpha * lapMac;
   if (x >= g.nx - 1) mac.x = 0.0f;
   if (z >= g.nz - 1) mac.z = 0.0f;
-  if (!ref && y >= g.ny - 1) mac.y = 0.0f;
+  if (y >= g.ny - 1) mac.y = 0.0f;
   stf(uo + i, mac.x); stf(vo + i, mac.y); stf(wo + i, mac.z);
 }
 
@@ -1161,16 +1196,27 @@ void launch_curl(const DevState& s, cudaStream_t st) {
   });
 }
 
+constexpr int kCassonRefZ = 4;  // planes per thread: 30 us at 96x128x96 (2: 31.7, 8: 37)
 void launch_casson(const DevState& s, cudaStream_t st, bool sparse) {
   // the samples' reach is worked out for whole dye cells per velocity cell
   const int r = s.gc.nx / s.g.nx;
   const bool whole = s.gc.nx == r * s.g.nx && s.gc.ny == r * s.g.ny && s.gc.nz == r * s.g.nz;
   const uint32_t* held = sparse && s.ref && whole ? held_flags_of(s, s.conc) : nullptr;
   DOB_VEL_DISPATCH(s.prec, {
-    k_casson<VS, DS><<<cell_grid(s.g), cell_block(), 0, st>>>(
-        s.g, s.gc, s.params, s.ref, s.flags, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w,
-        (const typename Vec4Of<VS>::type*)s.curl, (const typename Vec4Of<DS>::type*)s.conc, (const DS*)s.conc,
-        held, (VS*)s.u2, (VS*)s.v2, (VS*)s.w2);
+    auto run = [&](auto* k, int zc) {
+      k<<<col_grid(s.g, zc), cell_block(), 0, st>>>(
+          s.g, s.gc, s.params, s.flags, (const VS*)s.u, (const VS*)s.v, (const VS*)s.w,
+          (const typename Vec4Of<VS>::type*)s.curl, (const typename Vec4Of<DS>::type*)s.conc, held, (VS*)s.u2,
+          (VS*)s.v2, (VS*)s.w2);
+    };
+    if (!s.ref)
+      k_casson<VS, DS><<<cell_grid(s.g), cell_block(), 0, st>>>(s.g, s.gc, s.params, (const VS*)s.u, (const VS*)s.v,
+                                                                (const VS*)s.w, (const DS*)s.conc, (VS*)s.u2,
+                                                                (VS*)s.v2, (VS*)s.w2);
+    else if (long_columns(s, kCassonRefZ))
+      run(k_casson_ref<VS, DS, kCassonRefZ>, kCassonRefZ);
+    else
+      run(k_casson_ref<VS, DS, kShortZ>, kShortZ);
   });
 }
 
