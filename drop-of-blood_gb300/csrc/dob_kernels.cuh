@@ -51,6 +51,29 @@ __device__ __forceinline__ size_t brick_of(const Grid& gc, int x, int y, int z) 
 __device__ __forceinline__ bool brick_held(const Grid& gc, const uint32_t* flags, int x, int y, int z) {
   return !flags || __ldg(flags + brick_of(gc, x, y, z)) != 0u;
 }
+// Whether any brick overlapping the voxels [x0, x1] x [y0, y1] x [z0, z1]
+// (clamped to the grid) is flagged (arguments uniform over the block; every
+// thread must call it).
+__device__ __forceinline__ bool any_brick(const Grid& gc, const uint32_t* flags, int x0, int x1, int y0, int y1,
+                                          int z0, int z1) {
+  __shared__ int any;
+  const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
+  if (tid == 0) any = 0;
+  __syncthreads();
+  x0 = max(x0, 0); x1 = min(x1, gc.nx - 1);
+  y0 = max(y0, 0); y1 = min(y1, gc.ny - 1);
+  z0 = max(z0, 0); z1 = min(z1, gc.nz - 1);
+  const Grid b = brick_grid(gc);
+  const int bx0 = x0 / kDyeBrick, by0 = y0 / kDyeBrick, bz0 = z0 / kDyeBrick;
+  const int nbx = x1 / kDyeBrick - bx0 + 1, nby = y1 / kDyeBrick - by0 + 1, nbz = z1 / kDyeBrick - bz0 + 1;
+  const int count = nbx * nby * nbz;
+  for (int k = tid; k < count; k += blockDim.x * blockDim.y * blockDim.z) {
+    const int ix = k % nbx, iy = (k / nbx) % nby, iz = k / (nbx * nby);
+    if (__ldg(flags + b.at(bx0 + ix, by0 + iy, bz0 + iz))) any = 1;
+  }
+  __syncthreads();
+  return any != 0;
+}
 
 struct DevState {
   Grid g;    // velocity / pressure grid

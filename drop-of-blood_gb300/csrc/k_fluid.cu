@@ -334,30 +334,7 @@ constexpr float kDyeSpeedBound = 2.0f * 1.0001f;
 __device__ __forceinline__ void mark_brick(const Grid& gc, uint32_t* flags, int x, int y, int z) {
   flags[brick_of(gc, x, y, z)] = 1u;
 }
-// Whether any brick overlapping the voxels [x0, x1] x [y0, y1] x [z0, z1]
-// (clamped to the grid) is flagged (arguments uniform over the block; every
-// thread must call it).
-__device__ __forceinline__ bool any_brick(const Grid& gc, const uint32_t* flags, int x0, int x1, int y0, int y1,
-                                          int z0, int z1) {
-  __shared__ int any;
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-  if (tid == 0) any = 0;
-  __syncthreads();
-  x0 = max(x0, 0); x1 = min(x1, gc.nx - 1);
-  y0 = max(y0, 0); y1 = min(y1, gc.ny - 1);
-  z0 = max(z0, 0); z1 = min(z1, gc.nz - 1);
-  const Grid b = brick_grid(gc);
-  const int bx0 = x0 / kDyeBrick, by0 = y0 / kDyeBrick, bz0 = z0 / kDyeBrick;
-  const int nbx = x1 / kDyeBrick - bx0 + 1, nby = y1 / kDyeBrick - by0 + 1, nbz = z1 / kDyeBrick - bz0 + 1;
-  const int count = nbx * nby * nbz;
-  for (int k = tid; k < count; k += blockDim.x * blockDim.y) {
-    const int ix = k % nbx, iy = (k / nbx) % nby, iz = k / (nbx * nby);
-    if (__ldg(flags + b.at(bx0 + ix, by0 + iy, bz0 + iz))) any = 1;
-  }
-  __syncthreads();
-  return any != 0;
-}
-// The same for the block's voxels (x and y from the block index, planes
+// any_brick for the block's voxels (x and y from the block index, planes
 // zlo..zhi), widened by rx, ry, rz voxels per axis.
 __device__ __forceinline__ bool block_any_brick(const Grid& gc, const uint32_t* flags, int rx, int ry, int rz,
                                                 int zlo, int zhi) {

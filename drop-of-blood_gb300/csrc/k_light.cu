@@ -54,8 +54,19 @@ __device__ __forceinline__ float march(const Grid& gc, const V4* conc, dob_v3 uv
 template <class DS>
 __global__ void __launch_bounds__(kLightBX * kLightBY * kLightBZ)
     k_light_volume(Grid g, Grid gc, const StepParams* __restrict__ Pp,
-                   const typename Vec4Of<DS>::type* __restrict__ conc, const float4* __restrict__ wave,
-                   half4* __restrict__ light, float* __restrict__ brick_raw) {
+                   const typename Vec4Of<DS>::type* __restrict__ conc, const uint32_t* __restrict__ held,
+                   const float4* __restrict__ wave, half4* __restrict__ light, float* __restrict__ brick_raw) {
+  // held: the dye's brick flags.  A cell's five taps reach 1.02 cells from its
+  // centre, r dye voxels per cell, and a voxel more for the interpolation; in a
+  // block without dye there they are all +0 and the cell is clear (96x128x96
+  // with one plume: 67 -> 29 us, the dye's 148 MB from DRAM before).
+  bool dyed = true;
+  if (held) {
+    const int r = gc.nx / g.nx, m = 2 * r + 2;
+    const int x0 = blockIdx.x * kLightBX * r, y0 = blockIdx.y * kLightBY * r, z0 = blockIdx.z * kLightBZ * r;
+    dyed = any_brick(gc, held, x0 - m, x0 + kLightBX * r + m, y0 - m, y0 + kLightBY * r + m, z0 - m,
+                     z0 + kLightBZ * r + m);
+  }
   const int x = blockIdx.x * kLightBX + threadIdx.x;
   const int y = blockIdx.y * kLightBY + threadIdx.y;
   const int z = blockIdx.z * kLightBZ + threadIdx.z;
@@ -68,7 +79,7 @@ __global__ void __launch_bounds__(kLightBX * kLightBY * kLightBZ)
     const dob_v3 uvw = (v3((float)x, (float)y, (float)z) + v3(0.5f, 0.5f, 0.5f)) / dims;
     const dob_v3 p = to_world(P, uvw);
     const dob_v3 dom = dsize_of(P);
-    if (!(dob_maxf(fabsf(p.x), fabsf(p.z)) > 0.462f)) {
+    if (dyed && !(dob_maxf(fabsf(p.x), fabsf(p.z)) > 0.462f)) {
       // centre tap plus a tetrahedron of taps 1.02 voxels out (lighting.ts:47-58)
       const dob_v3 e = v3(1.02f, 1.02f, 1.02f) / dims;
       const float4 cC = lerp8x4(make_taps(gc, uvw.x, uvw.y, uvw.z), conc);
@@ -183,8 +194,12 @@ bool light_dims_ok(const Grid& g) { return g.nx % 4 == 0 && g.ny % 4 == 0 && g.n
 void launch_light_volume(const DevState& s, cudaStream_t st) {
   const dim3 block(kLightBX, kLightBY, kLightBZ);
   const dim3 grid((s.g.nx + kLightBX - 1) / kLightBX, s.g.ny / kLightBY, s.g.nz / kLightBZ);
+  // the taps' reach is worked out for whole dye cells per velocity cell
+  const int r = s.gc.nx / s.g.nx;
+  const bool whole = s.gc.nx == r * s.g.nx && s.gc.ny == r * s.g.ny && s.gc.nz == r * s.g.nz;
+  const uint32_t* held = whole ? held_flags_of(s, s.conc) : nullptr;
   DOB_VEL_DISPATCH(s.prec, k_light_volume<DS><<<grid, block, 0, st>>>(
-                               s.g, s.gc, s.params, static_cast<const typename Vec4Of<DS>::type*>(s.conc), s.wave,
+                               s.g, s.gc, s.params, static_cast<const typename Vec4Of<DS>::type*>(s.conc), held, s.wave,
                                s.light, s.brick_raw));
   const Grid b{s.g.nx / 4, s.g.ny / 4, s.g.nz / 4};
   k_brick_dilate<<<(unsigned)((b.n() + 255) / 256), 256, 0, st>>>(b, s.brick_raw, s.bricks);

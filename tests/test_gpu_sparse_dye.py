@@ -113,3 +113,27 @@ def test_reference_mode(dims, half):
     _run(sims, abi, True, dye, 3)
     _run(sims, abi, True, stages, 2)
     _run(sims, abi, True, lambda e: e.load_state(0), 3)
+
+
+@pytest.mark.parametrize("dims", [(24, 32, 24), (72, 40, 56)])
+def test_light_volume(dims):
+    from dropfluid import DropFluid, abi
+    from dropfluid.sequencer import SubstepSequencer
+    cfg = abi.config_reference()
+    cfg.nx, cfg.ny, cfg.nz = dims
+    cfg.mg_levels = 3
+    cfg.physics_flags = abi.DOB_PHYS_REFERENCE_ALL | abi.DOB_PHYS_LIGHTING
+    cfg.parcel_capacity = 49152
+    e = DropFluid(cfg)
+    seq = SubstepSequencer(parcel_capacity=cfg.parcel_capacity, seed=3.0)
+    e.set_uniforms(seq.reset_simulation(3.0, (0.05, -0.02)))
+    e.reset()
+    e.step_uniforms(np.stack([seq.advance_substep()[0] for _ in range(90)]))
+    got = []
+    for _ in range(2):  # the second with all flags set
+        e.bench_kernel(2, 1)  # the lighting passes on their own
+        got.append((e.get_field(abi.FIELD_LIGHT), e.get_field(abi.FIELD_BRICKS)))
+        e.set_field(abi.FIELD_CONC, e.get_field(abi.FIELD_CONC))
+    assert got[0][1].max() > 0
+    for x, y in zip(*got):
+        np.testing.assert_array_equal(x.view(np.uint32), y.view(np.uint32))
