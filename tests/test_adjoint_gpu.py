@@ -432,3 +432,27 @@ def test_mixed_gradient_directions_against_fp64_differences(gpu_lib, oracle_mod)
         assert rel_l2(grads["gpu"][k], grads["orc"][k]) < 3e-3, k
     g.close()
 
+
+
+@pytest.mark.parametrize("dims", [(16, 16, 16), (24, 32, 16)])
+def test_first_pressure_gradient_has_no_constant(gpu_lib, dims):
+    """The closed box's solve passes a constant through and removes the mean, so
+    d loss / d (first pressure) sums to zero over the black cells, which carry
+    it (the first half-sweep overwrites the red ones).  Bound: the mean is taken
+    out in FP32, one rounding of 2^-24 of each value."""
+    from dropfluid import DropFluid, abi
+    from dropfluid.adjoint import DropTrajectory
+    c = abi.config_closed_box(*dims)
+    c.parcel_capacity = 64
+    sim = DropFluid(c)
+    shape = dims[::-1]
+    z, y, x = np.meshgrid(*[np.linspace(0, 2 * np.pi, n) for n in shape], indexing="ij")
+    sim.set_field(abi.FIELD_VEL_U, np.sin(x + y).astype(np.float32))
+    sim.set_field(abi.FIELD_CONC, (0.5 + 0.4 * np.cos(y) * np.sin(z)).astype(np.float32))
+    sim.run_stage(abi.STAGE_MAC_TO_CENTER)
+    traj = DropTrajectory(sim, 2)
+    traj.forward(3)
+    g = np.asarray(traj.backward(np.cos(x + 2 * z).astype(np.float32))["p"], np.float64)
+    black = g[(np.indices(shape).sum(0) & 1) == 1]
+    assert np.abs(black).max() > 0
+    assert abs(black.sum()) <= 2.0 ** -24 * np.abs(black).sum()
