@@ -2,9 +2,10 @@
 // advection, MAC->centre, curl, Casson viscosity + forces, divergence,
 // projection, and the dye/conc transport kernels.
 //
-// Each kernel is one HBM-bound pass over the grid (one thread per cell,
-// x-fastest warps so every field access is a coalesced row segment; the
-// trilinear gathers of the centre field are 16 B AoS loads).
+// Each kernel is one pass over the grid (one thread per cell, or z-columns or
+// a list of dye bricks where noted; x-fastest warps so every field access is a
+// coalesced row segment; the trilinear gathers of the centre field are 16 B
+// AoS loads).
 #include "dob_column.cuh"
 #include "dob_kernels.cuh"
 
