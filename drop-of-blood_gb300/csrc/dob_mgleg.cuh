@@ -8,9 +8,10 @@
 // leg's dependence (one cell per half-sweep, one for the residual) and runs
 // the half-sweeps on it, so blocks never wait for one another.  The halo's
 // cells are computed by several blocks; every one of them forms the same
-// value (same operations in the same order as k_rbgs_v4 /
-// k_residual_restrict2 / k_prolong_add2, rounded to the level's storage type
-// after each half-sweep), so the results are the bits of the launch chain.
+// value (same operations in the same order as the half-sweep kernel of the
+// level's rows, k_rbgs_v4 or k_rbgs_split, k_residual_restrict2 and
+// k_prolong_add2, rounded to the level's storage type after each
+// half-sweep), so the results are the bits of the launch chain.
 // A block reads its neighbours' cells, so the leg's result goes to another
 // array than its input.
 //
@@ -59,7 +60,10 @@ struct LegCol {
   unsigned q;            // x parity of colour 0's cell at index 0
   int lane[2];           // the lane of the outer x neighbour of a cell of x parity 0, 1
   // diagonal of the cells of x parity 0, 1 away from the z walls and next to
-  // one, with the reciprocals, and these or 0 for a diagonal of 6
+  // one, with the reciprocals, and these again or 0 where the half-sweep
+  // multiplies by 1/6 instead of dividing: k_rbgs_v4 (rows of a multiple of 8)
+  // at every diagonal of 6, k_rbgs_split at interior cells only, so that it
+  // divides by the 6 of the row below the Dirichlet top
   float d0[2], r0[2], c0[2], d1[2], r1[2], c1[2];
   uint32_t at, sz;       // offset of (k, y, plane zb) in a colour's half, plane stride
   __device__ __forceinline__ LegCol(const Grid& d, int ref) {
@@ -79,13 +83,14 @@ struct LegCol {
     lane[0] = (tid & 31) - 1;
     lane[1] = (tid & 31) + 1;
     const float dy = 6.0f - (y == 0 ? 1.0f : 0.0f) - (y == d.ny - 1 && !ref ? 1.0f : 0.0f);
+    const bool divides = ref && y == d.ny - 1 && d.nx % 8 != 0;
 #pragma unroll
     for (int p = 0; p < 2; ++p) {
       d0[p] = dy - (k == (p ? hx - 1 : 0) ? 1.0f : 0.0f);
       d1[p] = d0[p] - 1.0f;
       r0[p] = d0[p] == 6.0f ? 1.0f / 6.0f : d0[p] == 5.0f ? 1.0f / 5.0f : d0[p] == 4.0f ? 1.0f / 4.0f : 1.0f / 3.0f;
       r1[p] = d1[p] == 5.0f ? 1.0f / 5.0f : d1[p] == 4.0f ? 1.0f / 4.0f : d1[p] == 3.0f ? 1.0f / 3.0f : 1.0f / 2.0f;
-      c0[p] = d0[p] == 6.0f ? 0.0f : r0[p];
+      c0[p] = d0[p] == 6.0f && !divides ? 0.0f : r0[p];
       c1[p] = r1[p];
     }
     sz = (uint32_t)d.ny * hx;
@@ -139,15 +144,19 @@ __device__ __forceinline__ float leg_sum(const LegCol<L>& t, LegShared<L>& sh, c
 // t / diag as the half-sweep kernels form it at colour c's cell of index i:
 // the product with 1/6, else the IEEE quotient (from the correctly rounded
 // reciprocal and one exact remainder, see div_by; an infinite quotient as it
-// is), rounded to the storage type; 0 outside the grid
+// is), rounded to the storage type; 0 outside the grid.  sixth: the product
+// at every diagonal of 6, as a restriction kernel forms the first red
+// half-sweep (restrict_pair)
 template <class T, class L>
-__device__ __forceinline__ float leg_value(const Grid& d, const LegCol<L>& t, int c, int i, float num) {
+__device__ __forceinline__ float leg_value(const Grid& d, const LegCol<L>& t, int c, int i, float num,
+                                           bool sixth = false) {
   if (!t.has_z(d, i)) return 0.0f;  // uniform over the half block
   const bool w = t.wall_z(d, i);
   const bool p = t.par(c, i) != 0;
   const float dg = w ? (p ? t.d1[1] : t.d1[0]) : (p ? t.d0[1] : t.d0[0]);
   const float r = w ? (p ? t.r1[1] : t.r1[0]) : (p ? t.r0[1] : t.r0[0]);
-  const float rc = w ? (p ? t.c1[1] : t.c1[0]) : (p ? t.c0[1] : t.c0[0]);
+  float rc = w ? (p ? t.c1[1] : t.c1[0]) : (p ? t.c0[1] : t.c0[0]);
+  if (sixth && dg == 6.0f) rc = 0.0f;
   const float qv = __fmul_rn(num, r);
   const float v = __fmaf_rn(__fmaf_rn(-qv, dg, num), rc, qv);
   return t.in ? as_stored<T>(fabsf(qv) <= 3.4028234e38f ? v : qv) : 0.0f;
@@ -187,7 +196,7 @@ __device__ __forceinline__ void leg_store(const Grid& d, const LegCol<L>& t, con
 // residual of the black cells goes to res (the red ones, updated last, have
 // none but rounding).
 template <class T, class TC, class L, bool ZERO, bool TR>
-__global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, float inv_h2, int ref,
+__global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, float inv_h2, int ref, int sixth,
                                                     const T* __restrict__ a, const T* __restrict__ b,
                                                     T* __restrict__ out, TC* __restrict__ bc, T* __restrict__ res,
                                                     const unsigned int* __restrict__ skip) {
@@ -207,7 +216,7 @@ __global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, f
     leg_load<T, L>(d, t, b, 0, bb[0]);
     leg_load<T, L>(d, t, b, 1, bb[1]);
 #pragma unroll
-    for (int i = 0; i < kLegZ; ++i) e[c0][i] = leg_value<T, L>(d, t, c0, i, 0.0f - h2 * bb[c0][i]);
+    for (int i = 0; i < kLegZ; ++i) e[c0][i] = leg_value<T, L>(d, t, c0, i, 0.0f - h2 * bb[c0][i], sixth != 0);
   } else {
     leg_load<T, L>(d, t, a, c0, e[c0]);
   }

@@ -87,8 +87,9 @@ __device__ __forceinline__ float rb_at(const T* a, const Grid& d, int x, int y, 
 
 // One colour of RBGS (createMgRbgsShader, fluid.ts:605-681), in place.
 // zoth: the other colour is zero (the first half-sweep from a zero guess), so
-// its values are not read; the result has the same bits as with zeroed
-// memory.
+// its values are not read; 1: the result has the same bits as with zeroed
+// memory; 2: as a restriction kernel forms it (restrict_pair: the product with
+// 1/6 at every diagonal of 6, the row below a Dirichlet top among them).
 template <class T>
 __global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2, int ref, int zoth,
                                                     T* __restrict__ a, const T* __restrict__ b,
@@ -114,7 +115,7 @@ __global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2,
     const float diag = (ref ? 1.0f : 0.0f) + (x > 0 ? 1.0f : 0.0f) + (x < d.nx - 1 ? 1.0f : 0.0f) +
                        (y > 0 ? 1.0f : 0.0f) + ((y < d.ny - 1 && !ref) ? 1.0f : 0.0f) + (z > 0 ? 1.0f : 0.0f) +
                        (z < d.nz - 1 ? 1.0f : 0.0f);
-    val = in ? (0.0f - h2 * bv) * (1.0f / 6.0f) : (0.0f - h2 * bv) / diag;
+    val = in || (zoth == 2 && diag == 6.0f) ? (0.0f - h2 * bv) * (1.0f / 6.0f) : (0.0f - h2 * bv) / diag;
   } else if (x > 0 && x < d.nx - 1 && y > 0 && y < d.ny - 1 && z > 0 && z < d.nz - 1) {
     // interior: six neighbours, diagonal 6 in both boundary modes
     const size_t sz = (size_t)d.ny * hx;
@@ -1413,9 +1414,10 @@ template <class T, class TC, class L>
 static void leg_down_l(const DevState& s, int l, const T* a, const T* b, T* out, TC* bc, T* res,
                        const unsigned int* skip, cudaStream_t st) {
   const MgLevel& V = s.lv[l];
+  const int sixth = s.prec != DOB_PREC_MIXED;
   auto run = [&](auto* k) {
-    launch_pdl(k, leg_grid<L>(V.d), dim3(L::NT), 0, st, V.d, s.lv[l + 1].d, V.h2, 1.0f / V.h2, s.ref, a, b, out, bc,
-               res, skip);
+    launch_pdl(k, leg_grid<L>(V.d), dim3(L::NT), 0, st, V.d, s.lv[l + 1].d, V.h2, 1.0f / V.h2, s.ref, sixth, a, b, out,
+               bc, res, skip);
   };
   if constexpr (sizeof(T) == 4 && sizeof(TC) == 4) {
     if (res) run(k_leg_down<T, TC, L, true, true>);
@@ -1506,7 +1508,8 @@ void launch_sumsq(const float* a, size_t n, double* out, int num_sms, cudaStream
 // leaves two waves of 1024 threads per SM (measured at 192x256x192: 20.5 us
 // per red+black pass with 2 planes against 24.6 us with 1; at 96x128x96 one
 // plane per thread is fastest).  Every level has even dims, so nz % 2 == 0.
-// zoth: the other colour is zero and is not read.
+// zoth: the other colour is zero and is not read (2: k_rbgs_split's second
+// form, which is k_rbgs_v4's only one).
 template <class T, bool ZOTH>
 static void half_sweep_v4(const DevState& s, const MgLevel& L, int c, T* own, const T* oth, const T* bown,
                           const unsigned int* skip, cudaStream_t st) {
@@ -1524,11 +1527,11 @@ static void half_sweep_v4(const DevState& s, const MgLevel& L, int c, T* own, co
   }
 }
 template <class T>
-static void half_sweep(const DevState& s, int l, int c, bool zoth, T* a, const T* b, const unsigned int* skip,
+static void half_sweep(const DevState& s, int l, int c, int zoth, T* a, const T* b, const unsigned int* skip,
                        cudaStream_t st) {
   const MgLevel& L = s.lv[l];
   if (L.d.nx % 8 != 0) {
-    launch_pdl(k_rbgs_split<T>, g_half(L.d), b_cells(), 0, st, L.d, c, L.h2, s.ref, zoth ? 1 : 0, a, b, skip);
+    launch_pdl(k_rbgs_split<T>, g_half(L.d), b_cells(), 0, st, L.d, c, L.h2, s.ref, zoth, a, b, skip);
     return;
   }
   const size_t half = L.d.n() >> 1;
@@ -1542,12 +1545,13 @@ static void half_sweep(const DevState& s, int l, int c, bool zoth, T* a, const T
 // `sweeps` red-black sweeps on level l, in place.  zero_first: the input is
 // zero (the first red half-sweep then reads no neighbours, and the black
 // half-sweep never reads its own old values, so nothing is filled unless
-// there are no sweeps); ec: coarse correction to add first.
+// there are no sweeps; 2: its first red half-sweep as a restriction would have
+// formed it, after one that did not); ec: coarse correction to add first.
 // red_done: the first red half-sweep from zero was formed by the restriction
 // into this level (restrict_level's ered)
 // flip: black before red (the transposed sweeps)
 template <class T, class TC = T>
-static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, bool zero_first, const TC* ec,
+static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, int zero_first, const TC* ec,
                    const unsigned int* skip, cudaStream_t st, bool red_done = false, int flip = 0) {
   const MgLevel& L = s.lv[l];
   if (zero_first && sweeps == 0) launch_pdl(k_fill_zero<T>, dim3(s.num_sms * 2), dim3(256), 0, st, a, L.d.n(), skip);
@@ -1572,7 +1576,7 @@ static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, bool 
   for (int k = 0; k < sweeps; ++k)
     for (int c = 0; c < 2; ++c) {
       if (red_done && k == 0 && c == 0) continue;
-      half_sweep<T>(s, l, c ^ flip, zero_first && k == 0 && c == 0, a, b, skip, st);
+      half_sweep<T>(s, l, c ^ flip, k == 0 && c == 0 ? zero_first : 0, a, b, skip, st);
     }
 }
 
@@ -1616,7 +1620,7 @@ static void vcycle(const DevState& s, T* x0, const T* b0, T* const* E, T* const*
   bool red_done = false;  // the restriction into the next level formed its red half-sweep
   const bool leg0 = leg_ok(s, 0) && !zero0;
   if (leg0) {
-    half_sweep<T>(s, 0, 0, false, x0, b0, skip, st);
+    half_sweep<T>(s, 0, 0, 0, x0, b0, skip, st);
     leg_down<T, T>(s, 0, x0, b0, s.lv[0].e2, B[1], s.pre0, skip, st);
   } else {
     smooth<T, T>(s, 0, x0, b0, s.pre0, zero0, nullptr, skip, st);
@@ -1631,7 +1635,7 @@ static void vcycle(const DevState& s, T* x0, const T* b0, T* const* E, T* const*
       X[l] = s.lv[l].e2;
       red_done = false;
     } else {
-      smooth<T, T>(s, l, E[l], B[l], s.pre, true, nullptr, skip, st, red_done);
+      smooth<T, T>(s, l, E[l], B[l], s.pre, 2, nullptr, skip, st, red_done);
       restrict_level<T>(s, l, E[l], B[l], B[l + 1], skip, st, nullptr, nullptr, ered(l + 1));
       red_done = ered(l + 1) != nullptr;
     }
