@@ -90,8 +90,9 @@ __device__ __forceinline__ float rb_at(const T* a, const Grid& d, int x, int y, 
 // its values are not read; 1: the result has the same bits as with zeroed
 // memory; 2: as a restriction kernel forms it (restrict_pair: the product with
 // 1/6 at every diagonal of 6, the row below a Dirichlet top among them).
+// six: 6, or 0 to divide by every diagonal (zoth 0 or 1).
 template <class T>
-__global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2, int ref, int zoth,
+__global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2, int ref, int zoth, float six,
                                                     T* __restrict__ a, const T* __restrict__ b,
                                                     const unsigned int* __restrict__ skip) {
   pdl_wait();
@@ -115,13 +116,13 @@ __global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2,
     const float diag = (ref ? 1.0f : 0.0f) + (x > 0 ? 1.0f : 0.0f) + (x < d.nx - 1 ? 1.0f : 0.0f) +
                        (y > 0 ? 1.0f : 0.0f) + ((y < d.ny - 1 && !ref) ? 1.0f : 0.0f) + (z > 0 ? 1.0f : 0.0f) +
                        (z < d.nz - 1 ? 1.0f : 0.0f);
-    val = in || (zoth == 2 && diag == 6.0f) ? (0.0f - h2 * bv) * (1.0f / 6.0f) : (0.0f - h2 * bv) / diag;
+    val = (in && diag == six) || (zoth == 2 && diag == 6.0f) ? (0.0f - h2 * bv) * (1.0f / 6.0f) : (0.0f - h2 * bv) / diag;
   } else if (x > 0 && x < d.nx - 1 && y > 0 && y < d.ny - 1 && z > 0 && z < d.nz - 1) {
     // interior: six neighbours, diagonal 6 in both boundary modes
     const size_t sz = (size_t)d.ny * hx;
     const float sumN = ((((ldv(oth + r + ((x - 1) >> 1)) + ldv(oth + r + ((x + 1) >> 1))) + ldv(oth + i - hx)) +
                          ldv(oth + i + hx)) + ldv(oth + i - sz)) + ldv(oth + i + sz);
-    val = (sumN - h2 * bv) * (1.0f / 6.0f);
+    val = six == 6.0f ? (sumN - h2 * bv) * (1.0f / 6.0f) : (sumN - h2 * bv) / 6.0f;
   } else {
     float sumN, diag;
     stencil_rb(oth, d, x, y, z, r, k, ref, sumN, diag);
@@ -178,8 +179,9 @@ __device__ __forceinline__ float f4get(const float4& v, int j) {
 // Offsets are 32-bit (split halves have fewer than 2^30 words).  `own` and
 // `oth` are the two halves of the level's array (disjoint).  ZOTH: the other
 // colour is zero (first half-sweep from a zero guess) and is not read.
+// six: 6, or 0 to divide by every diagonal.
 template <class T, int ZC, bool ZOTH>
-__global__ void __launch_bounds__(256) k_rbgs_v4(Grid d, int color, float h2, int ref, T* __restrict__ own,
+__global__ void __launch_bounds__(256) k_rbgs_v4(Grid d, int color, float h2, int ref, float six, T* __restrict__ own,
                                                  const T* __restrict__ oth, const T* __restrict__ bown,
                                                  const unsigned int* __restrict__ skip) {
   pdl_wait();
@@ -236,7 +238,7 @@ __global__ void __launch_bounds__(256) k_rbgs_v4(Grid d, int color, float h2, in
       sumN = fmaf(wzp, f4get(zp, j), sumN);
       const float diag = dyz + (wxm + wxp);
       const float t = sumN - h2 * f4get(bv, j);
-      res[j] = diag == 6.0f ? t * (1.0f / 6.0f) : t / diag;
+      res[j] = diag == six ? t * (1.0f / 6.0f) : t / diag;
     }
     Vec4Ld<T>::st(own + r, make_float4(res[0], res[1], res[2], res[3]));
   }
@@ -814,6 +816,7 @@ __global__ void k_fill_zero(T* __restrict__ a, size_t n, const unsigned int* __r
 // where two CTAs that formed them from the index on every update took 31.
 constexpr int kCoarseThreads = 1024, kCoarseCells = 4;
 constexpr size_t kCoarseSmem = 220 * 1024;  // dynamic shared memory, at most
+constexpr size_t kCoarseSlab = 25600;       // see coarse_solve
 __host__ __device__ inline size_t coarse_words(const Grid& d, int cs) {  // shared floats per CTA
   const size_t pz = (d.nz + cs - 1) / cs, hx = d.nx / 2;
   return 2 * (hx + 2) * (d.ny + 2) * (pz + 2);
@@ -1509,37 +1512,39 @@ void launch_sumsq(const float* a, size_t n, double* out, int num_sms, cudaStream
 // per red+black pass with 2 planes against 24.6 us with 1; at 96x128x96 one
 // plane per thread is fastest).  Every level has even dims, so nz % 2 == 0.
 // zoth: the other colour is zero and is not read (2: k_rbgs_split's second
-// form, which is k_rbgs_v4's only one).
+// form, which is k_rbgs_v4's only one).  divide: by the diagonal at every cell,
+// as the kernels that sweep the coarsest grid in one launch do.
 template <class T, bool ZOTH>
-static void half_sweep_v4(const DevState& s, const MgLevel& L, int c, T* own, const T* oth, const T* bown,
+static void half_sweep_v4(const DevState& s, const MgLevel& L, int c, float six, T* own, const T* oth, const T* bown,
                           const unsigned int* skip, cudaStream_t st) {
   const dim3 bq = quad_block(L.d);
   dim3 gq = quad_grid(L.d, bq);
   const size_t threads = (L.d.n() >> 1) / 4, wave2 = (size_t)s.num_sms * 2048;
   if (L.d.nz % 4 == 0 && threads / 4 >= wave2) {
     gq.z = L.d.nz / 4;
-    launch_pdl(k_rbgs_v4<T, 4, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
+    launch_pdl(k_rbgs_v4<T, 4, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, six, own, oth, bown, skip);
   } else if (threads / 2 >= wave2) {
     gq.z = L.d.nz / 2;
-    launch_pdl(k_rbgs_v4<T, 2, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
+    launch_pdl(k_rbgs_v4<T, 2, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, six, own, oth, bown, skip);
   } else {
-    launch_pdl(k_rbgs_v4<T, 1, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
+    launch_pdl(k_rbgs_v4<T, 1, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, six, own, oth, bown, skip);
   }
 }
 template <class T>
 static void half_sweep(const DevState& s, int l, int c, int zoth, T* a, const T* b, const unsigned int* skip,
-                       cudaStream_t st) {
+                       cudaStream_t st, bool divide = false) {
   const MgLevel& L = s.lv[l];
+  const float six = divide ? 0.0f : 6.0f;
   if (L.d.nx % 8 != 0) {
-    launch_pdl(k_rbgs_split<T>, g_half(L.d), b_cells(), 0, st, L.d, c, L.h2, s.ref, zoth, a, b, skip);
+    launch_pdl(k_rbgs_split<T>, g_half(L.d), b_cells(), 0, st, L.d, c, L.h2, s.ref, zoth, six, a, b, skip);
     return;
   }
   const size_t half = L.d.n() >> 1;
   T* own = a + (c ? half : 0);
   const T* oth = a + (c ? 0 : half);
   const T* bown = b + (c ? half : 0);
-  if (zoth) half_sweep_v4<T, true>(s, L, c, own, oth, bown, skip, st);
-  else half_sweep_v4<T, false>(s, L, c, own, oth, bown, skip, st);
+  if (zoth) half_sweep_v4<T, true>(s, L, c, six, own, oth, bown, skip, st);
+  else half_sweep_v4<T, false>(s, L, c, six, own, oth, bown, skip, st);
 }
 
 // `sweeps` red-black sweeps on level l, in place.  zero_first: the input is
@@ -1549,10 +1554,11 @@ static void half_sweep(const DevState& s, int l, int c, int zoth, T* a, const T*
 // formed it, after one that did not); ec: coarse correction to add first.
 // red_done: the first red half-sweep from zero was formed by the restriction
 // into this level (restrict_level's ered)
-// flip: black before red (the transposed sweeps)
+// flip: black before red (the transposed sweeps); divide: see half_sweep
 template <class T, class TC = T>
 static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, int zero_first, const TC* ec,
-                   const unsigned int* skip, cudaStream_t st, bool red_done = false, int flip = 0) {
+                   const unsigned int* skip, cudaStream_t st, bool red_done = false, int flip = 0,
+                   bool divide = false) {
   const MgLevel& L = s.lv[l];
   if (zero_first && sweeps == 0) launch_pdl(k_fill_zero<T>, dim3(s.num_sms * 2), dim3(256), 0, st, a, L.d.n(), skip);
   if (ec) {
@@ -1576,7 +1582,7 @@ static void smooth(const DevState& s, int l, T* a, const T* b, int sweeps, int z
   for (int k = 0; k < sweeps; ++k)
     for (int c = 0; c < 2; ++c) {
       if (red_done && k == 0 && c == 0) continue;
-      half_sweep<T>(s, l, c ^ flip, k == 0 && c == 0 ? zero_first : 0, a, b, skip, st);
+      half_sweep<T>(s, l, c ^ flip, k == 0 && c == 0 ? zero_first : 0, a, b, skip, st, divide);
     }
 }
 
@@ -1592,14 +1598,23 @@ static void coarse_solve(const DevState& s, int l, T* e, const T* b, const unsig
                  s.cinv, s.cn, e, b, skip);
     return;
   }
-  // one CTA where its threads hold the grid, else a cluster of eight
+  // Grids of up to kCoarseSlab cells for each of 8, 4 or 2 slabs of whole planes
+  // divide by the diagonal at every cell, larger ones smooth as the other
+  // levels do: the pressure's last bits hang on the line, so it stays where
+  // recorded runs have it.  The dividing sweeps run in one CTA where its threads
+  // hold the grid, else in a cluster of eight that do, else half by half, the
+  // same bits (48x64x48 cells, six sweeps, four cycles: a step of 96x128x96 on
+  // two grids takes 333 us; slabs in a cluster's shared memory, indices formed
+  // on every update: 821).
+  bool divide = false;
+  for (int c : {8, 4, 2}) divide = divide || (L.d.nz % c == 0 && L.d.n() / c <= kCoarseSlab);
   auto run = [&](auto* k, int cs) {
     launch_pdl(k, dim3(cs), dim3(kCoarseThreads), coarse_words(L.d, cs) * sizeof(float), st, L.d, L.h2, s.ref,
                s.coarse_sweeps, flip, e, b, skip);
   };
-  if (coarse_fits(L.d, 1)) run(k_coarse_sweeps<T, 1>, 1);
-  else if (coarse_fits(L.d, 8)) run(k_coarse_sweeps<T, 8>, 8);
-  else smooth<T, T>(s, l, e, b, s.coarse_sweeps, true, nullptr, skip, st, false, flip);
+  if (divide && coarse_fits(L.d, 1)) run(k_coarse_sweeps<T, 1>, 1);
+  else if (divide && coarse_fits(L.d, 8)) run(k_coarse_sweeps<T, 8>, 8);
+  else smooth<T, T>(s, l, e, b, s.coarse_sweeps, true, nullptr, skip, st, false, flip, divide);
 }
 
 // One V-cycle on (x0, b0); per-level arrays E[l], B[l] for l >= 1.
