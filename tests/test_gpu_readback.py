@@ -25,3 +25,41 @@ def test_fields_come_back_as_stored(dims, mixed):
     np.testing.assert_array_equal(sim.get_field(abi.FIELD_PRESSURE), p)
     stored = dye.astype(np.float16).astype(np.float32) if mixed else dye
     np.testing.assert_array_equal(sim.get_field(abi.FIELD_CONC), stored)
+
+
+def test_reading_into_a_used_buffer_costs_the_copy(gpu_lib):
+    """A buffer that has its pages is not populated again: one call over 256 MB
+    takes no longer than forty calls over its pieces of less than 8 MB, which
+    are never populated."""
+    import ctypes
+    import time
+    from dropfluid import DropFluid, abi
+    cfg = abi.config_closed_box(16, 16, 16)
+    n, pieces = 8000000, 40
+    cfg.parcel_capacity = n
+    sim = DropFluid(cfg)
+    out = np.zeros((n, abi.PARCEL_FLOATS), np.float32)
+    out += 1.0  # backed with memory
+
+    def read(first, count):
+        p = out[first:].ctypes.data_as(ctypes.POINTER(ctypes.c_float))
+        assert gpu_lib.dob_get_parcels(sim._h, p, count, first) == 0
+
+    def whole():
+        read(0, n)
+
+    def parts():
+        for k in range(pieces):
+            read(k * (n // pieces), n // pieces)
+
+    def best(f):
+        times = []
+        for _ in range(20):
+            t = time.perf_counter()
+            f()
+            times.append(time.perf_counter() - t)
+        return min(times)
+
+    best(parts)
+    assert best(whole) <= best(parts)
+    sim.close()
