@@ -175,7 +175,7 @@ def run_scene_steps(scene, eng, start, n, timed, graph=True):
         if timed:
             total += eng.time_steps(seg)
         else:
-            eng.step(seg, graph=graph)
+            eng.step(seg, **({} if graph else {"graph": False}))  # the oracle's step has no graph
         k = nxt
     return total
 
