@@ -149,7 +149,6 @@ struct AdjState {
   float *alpha, *gq;       // Casson adjoint scratch: per-cell alpha, 2 dL/dQ (and the transposed cycle's)
   double* part;            // partial sums of the mean removals: 2 x kSumBlocks
   float *lam, *lamlo;      // mixed mode: adjoint pressure solve's solution pair (split)
-  double* red;             // FP64 reduction slots (mean removal)
 };
 // relative residual of the mixed mode's adjoint pressure solve
 constexpr double kAdjRelTol = 1e-6;

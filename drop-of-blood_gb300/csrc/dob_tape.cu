@@ -135,7 +135,6 @@ dob_status ensure_adj(dob_ctx* ctx) {
   if (s.prec == DOB_PREC_MIXED) { F(&a.lam, N); F(&a.lamlo, N); }
   if (s.prec != DOB_PREC_MIXED)
     for (int l = 1; l < s.nlev; ++l) F(&a.lr[l], s.lv[l].d.n());
-  if (st == DOB_OK) st = alloc(ctx, A->bufs, (void**)&a.red, 8 * sizeof(double));
   if (st == DOB_OK) st = alloc(ctx, A->bufs, (void**)&a.part, 2 * kSumBlocks * sizeof(double));
   if (st == DOB_OK) st = alloc(ctx, A->bufs, (void**)&A->dred, 4 * sizeof(double));
   if (st != DOB_OK) adjoint_free(ctx);
@@ -516,7 +515,7 @@ dob_status dob_tape_backward(dob_ctx* ctx, const float* dye_grad, size_t bytes) 
   // is taken out: two passes over half a grid, 10 us a backward pass.
   const size_t half = s.g.n() >> 1;
   const int sweeps = s.nlev == 1 ? s.pre + s.post : s.pre0;
-  if (!mixed(ctx) && s.cycles > 0 && sweeps > 0 && half % 4 == 0) {  // 16-byte loads
+  if (!mixed(ctx) && s.cycles > 0 && sweeps > 0) {  // (all dims are even: half is a multiple of 4)
     launch_sum(A->a.ap + half, half, A->a.part, s.num_sms, st);
     launch_sub_mean(A->a.ap + half, half, A->a.part, s.num_sms, st);
   }

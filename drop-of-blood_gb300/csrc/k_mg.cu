@@ -79,12 +79,6 @@ __device__ __forceinline__ void stencil_rb(const T* oth, const Grid& d, int x, i
   if (z < d.nz - 1) { sumN = sumN + ldv(oth + r + (size_t)d.ny * hx + k); diag = diag + 1.0f; }
 }
 
-// Value of the split array at natural coordinates.
-template <class T>
-__device__ __forceinline__ float rb_at(const T* a, const Grid& d, int x, int y, int z) {
-  return ldv(a + rb_index(d, x, y, z));
-}
-
 // One colour of RBGS (createMgRbgsShader, fluid.ts:605-681), in place.
 // zoth: the other colour is zero (the first half-sweep from a zero guess), so
 // its values are not read; 1: the result has the same bits as with zeroed
