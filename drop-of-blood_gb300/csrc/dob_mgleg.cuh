@@ -144,19 +144,15 @@ __device__ __forceinline__ float leg_sum(const LegCol<L>& t, LegShared<L>& sh, c
 // t / diag as the half-sweep kernels form it at colour c's cell of index i:
 // the product with 1/6, else the IEEE quotient (from the correctly rounded
 // reciprocal and one exact remainder, see div_by; an infinite quotient as it
-// is), rounded to the storage type; 0 outside the grid.  sixth: the product
-// at every diagonal of 6, as a restriction kernel forms the first red
-// half-sweep (restrict_pair)
+// is), rounded to the storage type; 0 outside the grid
 template <class T, class L>
-__device__ __forceinline__ float leg_value(const Grid& d, const LegCol<L>& t, int c, int i, float num,
-                                           bool sixth = false) {
+__device__ __forceinline__ float leg_value(const Grid& d, const LegCol<L>& t, int c, int i, float num) {
   if (!t.has_z(d, i)) return 0.0f;  // uniform over the half block
   const bool w = t.wall_z(d, i);
   const bool p = t.par(c, i) != 0;
   const float dg = w ? (p ? t.d1[1] : t.d1[0]) : (p ? t.d0[1] : t.d0[0]);
   const float r = w ? (p ? t.r1[1] : t.r1[0]) : (p ? t.r0[1] : t.r0[0]);
-  float rc = w ? (p ? t.c1[1] : t.c1[0]) : (p ? t.c0[1] : t.c0[0]);
-  if (sixth && dg == 6.0f) rc = 0.0f;
+  const float rc = w ? (p ? t.c1[1] : t.c1[0]) : (p ? t.c0[1] : t.c0[0]);
   const float qv = __fmul_rn(num, r);
   const float v = __fmaf_rn(__fmaf_rn(-qv, dg, num), rc, qv);
   return t.in ? as_stored<T>(fabsf(qv) <= 3.4028234e38f ? v : qv) : 0.0f;
@@ -195,6 +191,9 @@ __device__ __forceinline__ void leg_store(const Grid& d, const LegCol<L>& t, con
 // TR (with ZERO; the transposed cycle): the colours change places, and the
 // residual of the black cells goes to res (the red ones, updated last, have
 // none but rounding).
+// sixth (with ZERO): the first half-sweep multiplies by 1/6 at every diagonal of
+// 6, as the restriction forms it in the FP32 cycle's chain (restrict_pair); in
+// the mixed one's chain the half-sweep kernel forms it.
 template <class T, class TC, class L, bool ZERO, bool TR>
 __global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, float inv_h2, int ref, int sixth,
                                                     const T* __restrict__ a, const T* __restrict__ b,
@@ -215,8 +214,12 @@ __global__ void __launch_bounds__(L::NT) k_leg_down(Grid d, Grid dc, float h2, f
   if (ZERO) {
     leg_load<T, L>(d, t, b, 0, bb[0]);
     leg_load<T, L>(d, t, b, 1, bb[1]);
+    LegCol<L> first = t;
 #pragma unroll
-    for (int i = 0; i < kLegZ; ++i) e[c0][i] = leg_value<T, L>(d, t, c0, i, 0.0f - h2 * bb[c0][i], sixth != 0);
+    for (int p = 0; p < 2; ++p)
+      if (sixth && t.d0[p] == 6.0f) first.c0[p] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kLegZ; ++i) e[c0][i] = leg_value<T, L>(d, first, c0, i, 0.0f - h2 * bb[c0][i]);
   } else {
     leg_load<T, L>(d, t, a, c0, e[c0]);
   }

@@ -84,9 +84,9 @@ __device__ __forceinline__ void stencil_rb(const T* oth, const Grid& d, int x, i
 // its values are not read; 1: the result has the same bits as with zeroed
 // memory; 2: as a restriction kernel forms it (restrict_pair: the product with
 // 1/6 at every diagonal of 6, the row below a Dirichlet top among them).
-// six: 6, or 0 to divide by every diagonal (zoth 0 or 1).
-template <class T>
-__global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2, int ref, int zoth, float six,
+// DIV: divides by every diagonal (zoth 0 or 1).
+template <class T, bool DIV>
+__global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2, int ref, int zoth,
                                                     T* __restrict__ a, const T* __restrict__ b,
                                                     const unsigned int* __restrict__ skip) {
   pdl_wait();
@@ -110,13 +110,13 @@ __global__ void __launch_bounds__(256) k_rbgs_split(Grid d, int color, float h2,
     const float diag = (ref ? 1.0f : 0.0f) + (x > 0 ? 1.0f : 0.0f) + (x < d.nx - 1 ? 1.0f : 0.0f) +
                        (y > 0 ? 1.0f : 0.0f) + ((y < d.ny - 1 && !ref) ? 1.0f : 0.0f) + (z > 0 ? 1.0f : 0.0f) +
                        (z < d.nz - 1 ? 1.0f : 0.0f);
-    val = (in && diag == six) || (zoth == 2 && diag == 6.0f) ? (0.0f - h2 * bv) * (1.0f / 6.0f) : (0.0f - h2 * bv) / diag;
+    val = (in && !DIV) || (zoth == 2 && diag == 6.0f) ? (0.0f - h2 * bv) * (1.0f / 6.0f) : (0.0f - h2 * bv) / diag;
   } else if (x > 0 && x < d.nx - 1 && y > 0 && y < d.ny - 1 && z > 0 && z < d.nz - 1) {
     // interior: six neighbours, diagonal 6 in both boundary modes
     const size_t sz = (size_t)d.ny * hx;
     const float sumN = ((((ldv(oth + r + ((x - 1) >> 1)) + ldv(oth + r + ((x + 1) >> 1))) + ldv(oth + i - hx)) +
                          ldv(oth + i + hx)) + ldv(oth + i - sz)) + ldv(oth + i + sz);
-    val = six == 6.0f ? (sumN - h2 * bv) * (1.0f / 6.0f) : (sumN - h2 * bv) / 6.0f;
+    val = DIV ? (sumN - h2 * bv) / 6.0f : (sumN - h2 * bv) * (1.0f / 6.0f);
   } else {
     float sumN, diag;
     stencil_rb(oth, d, x, y, z, r, k, ref, sumN, diag);
@@ -173,9 +173,10 @@ __device__ __forceinline__ float f4get(const float4& v, int j) {
 // Offsets are 32-bit (split halves have fewer than 2^30 words).  `own` and
 // `oth` are the two halves of the level's array (disjoint).  ZOTH: the other
 // colour is zero (first half-sweep from a zero guess) and is not read.
-// six: 6, or 0 to divide by every diagonal.
-template <class T, int ZC, bool ZOTH>
-__global__ void __launch_bounds__(256) k_rbgs_v4(Grid d, int color, float h2, int ref, float six, T* __restrict__ own,
+// DIV: divides by every diagonal (a template: a number to compare with, passed
+// in, cost box192's level-0 pass 20.7 -> 21.8 us).
+template <class T, int ZC, bool ZOTH, bool DIV = false>
+__global__ void __launch_bounds__(256) k_rbgs_v4(Grid d, int color, float h2, int ref, T* __restrict__ own,
                                                  const T* __restrict__ oth, const T* __restrict__ bown,
                                                  const unsigned int* __restrict__ skip) {
   pdl_wait();
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(256) k_rbgs_v4(Grid d, int color, float h2, in
       sumN = fmaf(wzp, f4get(zp, j), sumN);
       const float diag = dyz + (wxm + wxp);
       const float t = sumN - h2 * f4get(bv, j);
-      res[j] = diag == six ? t * (1.0f / 6.0f) : t / diag;
+      res[j] = !DIV && diag == 6.0f ? t * (1.0f / 6.0f) : t / diag;
     }
     Vec4Ld<T>::st(own + r, make_float4(res[0], res[1], res[2], res[3]));
   }
@@ -1509,36 +1510,39 @@ void launch_sumsq(const float* a, size_t n, double* out, int num_sms, cudaStream
 // form, which is k_rbgs_v4's only one).  divide: by the diagonal at every cell,
 // as the kernels that sweep the coarsest grid in one launch do.
 template <class T, bool ZOTH>
-static void half_sweep_v4(const DevState& s, const MgLevel& L, int c, float six, T* own, const T* oth, const T* bown,
+static void half_sweep_v4(const DevState& s, const MgLevel& L, int c, bool divide, T* own, const T* oth, const T* bown,
                           const unsigned int* skip, cudaStream_t st) {
   const dim3 bq = quad_block(L.d);
   dim3 gq = quad_grid(L.d, bq);
   const size_t threads = (L.d.n() >> 1) / 4, wave2 = (size_t)s.num_sms * 2048;
-  if (L.d.nz % 4 == 0 && threads / 4 >= wave2) {
+  if (divide) {  // the coarsest grid, at most 204800 cells
+    launch_pdl(k_rbgs_v4<T, 1, ZOTH, true>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
+  } else if (L.d.nz % 4 == 0 && threads / 4 >= wave2) {
     gq.z = L.d.nz / 4;
-    launch_pdl(k_rbgs_v4<T, 4, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, six, own, oth, bown, skip);
+    launch_pdl(k_rbgs_v4<T, 4, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
   } else if (threads / 2 >= wave2) {
     gq.z = L.d.nz / 2;
-    launch_pdl(k_rbgs_v4<T, 2, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, six, own, oth, bown, skip);
+    launch_pdl(k_rbgs_v4<T, 2, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
   } else {
-    launch_pdl(k_rbgs_v4<T, 1, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, six, own, oth, bown, skip);
+    launch_pdl(k_rbgs_v4<T, 1, ZOTH>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
   }
 }
 template <class T>
 static void half_sweep(const DevState& s, int l, int c, int zoth, T* a, const T* b, const unsigned int* skip,
                        cudaStream_t st, bool divide = false) {
   const MgLevel& L = s.lv[l];
-  const float six = divide ? 0.0f : 6.0f;
   if (L.d.nx % 8 != 0) {
-    launch_pdl(k_rbgs_split<T>, g_half(L.d), b_cells(), 0, st, L.d, c, L.h2, s.ref, zoth, six, a, b, skip);
+    auto run = [&](auto* k) { launch_pdl(k, g_half(L.d), b_cells(), 0, st, L.d, c, L.h2, s.ref, zoth, a, b, skip); };
+    if (divide) run(k_rbgs_split<T, true>);
+    else run(k_rbgs_split<T, false>);
     return;
   }
   const size_t half = L.d.n() >> 1;
   T* own = a + (c ? half : 0);
   const T* oth = a + (c ? 0 : half);
   const T* bown = b + (c ? half : 0);
-  if (zoth) half_sweep_v4<T, true>(s, L, c, six, own, oth, bown, skip, st);
-  else half_sweep_v4<T, false>(s, L, c, six, own, oth, bown, skip, st);
+  if (zoth) half_sweep_v4<T, true>(s, L, c, divide, own, oth, bown, skip, st);
+  else half_sweep_v4<T, false>(s, L, c, divide, own, oth, bown, skip, st);
 }
 
 // `sweeps` red-black sweeps on level l, in place.  zero_first: the input is
