@@ -12,8 +12,10 @@
 // projection use the z-column kernels of k_box.cu (same bits as the general
 // kernels the stage-level interface runs).  The stage sequence is
 // captured once into a CUDA graph per (dye, velocity) ping-pong state and
-// replayed; the per-step parameters reach the device by one 592-byte copy
-// from a pinned ring before each replay.
+// replayed; the per-step parameters reach the device by one 604-byte copy
+// from a pinned ring before each replay, and where the next step's wave
+// substep runs early (steps of one call, DOB_PHYS_WAVE) by one more of its
+// 512-byte uniform block.
 #include <cuda_runtime.h>
 #include <math.h>
 #include <stdio.h>

@@ -27,9 +27,9 @@
 // neighbours, hold values that nothing needed reads.  Cells outside the grid
 // are zeros that nothing updates, so absent neighbours add an exact zero.
 //
-// Measured (the step's graph, four 2+2 cycles): 48x64x48 234 -> 185 us a
-// step, of which the solve 180 -> 129; 192x256x192, whose levels 2 and 3 run
-// this way, 1326 -> 1289.  One thread per cell and half-sweep with index
+// Measured (four 2+2 cycles): 48x64x48 234 -> 185 us a step in the graph (the
+// solve as a stage 184 -> 135); 192x256x192, whose levels 2 and 3 run this way,
+// 1326 -> 1289.  One thread per cell and half-sweep with index
 // arithmetic (263 us a step) and one thread per whole z column (209) were
 // slower: the legs are bound by the instruction latency of their few warps.
 #pragma once

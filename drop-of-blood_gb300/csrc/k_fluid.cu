@@ -374,7 +374,7 @@ __device__ __forceinline__ dob_v3 sample_conc_rg(const Grid& gc, const typename 
 
 // Reference mode, on z-columns (dob_column.cuh): the same expressions in the
 // same order as one thread per cell formed them with 18 clamped loads around
-// it (630 instructions a warp; FIGURES).
+// it (630 instructions a warp): 34 -> 30 us at 96x128x96.
 // held (inside a step): the dye's flags.  The cell's two samples, at its
 // centre and on its upper y face, tap dye voxels r x - 1 to r (x + 1) per axis
 // (r dye cells per cell); one more for the rounding of the texel and 1/1000 of
@@ -1263,8 +1263,8 @@ void launch_dye_flags_begin(const DevState& s, cudaStream_t st) {
 // Lists from a million voxels: at 96x128x96 (1.2 million) the predictor takes
 // 14.9 us with the list and 18.2 without, at 72x104x56 (419 thousand) 11.1 and
 // 12.5 but the resolve 9.6 and 8.1 (steps 252 and 250 us): there the list's
-// launch costs what it saves.  The reference resolve, whose stage is heavier,
-// is always listed.
+// launch costs what it saves (where between the two the line lies was not
+// looked for).  The reference resolve, whose stage is heavier, is always listed.
 static bool dye_listed(const DevState& s) { return s.gc.n() >= 1000000u; }
 template <int MODE, class DS, int PER>
 static void launch_dye_list(const DevState& s, const uint32_t* flags, const uint32_t* old, const unsigned int* speed,

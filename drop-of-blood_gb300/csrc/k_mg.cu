@@ -1395,7 +1395,9 @@ void launch_split(const float* src, float* dst, const Grid& d, bool to_split, cu
 // Levels of up to half a million cells: there a leg's redundant halo work
 // costs less than the launches it saves (level of 72x104x56 = 419k cells:
 // 254 against 263 us a step); at 1.2 million (96x128x96) the launch chain,
-// which does no work twice, is faster (257 against 302 us a step).
+// which does no work twice, is faster (257 against 302 us a step).  Both with
+// two sweeps each way; the line between them, and one for single sweeps, whose
+// halo is smaller, were not looked for.
 constexpr size_t kLegMaxCells = 500000;
 bool mg_leg_level(const Grid& d) { return d.n() <= kLegMaxCells; }
 template <class L> static dim3 leg_grid(const Grid& d) {

@@ -368,10 +368,12 @@ dob_status dob_sync(dob_ctx* ctx);
 /* Kernels launched by one step (kernel nodes of the captured step graph). */
 dob_status dob_launches_per_step(dob_ctx* ctx, int* n);
 
-/* Host<->device bytes of one step through this ABI: the per-step parameter
-   block copied host->device before each step (steps of one dob_step_uniforms
-   call with the wave solver also copy the next step's block ahead), and the
-   statistics read back device->host by a dob_step with DOB_STEP_STATS. */
+/* Host<->device bytes of a call of one step through this ABI: the per-step
+   parameter block copied host->device before the step, and the statistics
+   read back device->host by a dob_step with DOB_STEP_STATS.  Not counted:
+   with the wave solver, every step but the last of a call of several
+   (dob_step_uniforms, dob_step, dob_time_steps) also copies the 512-byte
+   uniform block of the step after it. */
 dob_status dob_io_bytes(const dob_ctx* ctx, uint64_t* h2d_per_step, uint64_t* d2h_stats);
 
 /* Device memory held by this context, in bytes. */
