@@ -642,11 +642,36 @@ __global__ void __launch_bounds__(256) k_inject_t2(Grid f, Grid c, float* __rest
     Pair<float>::st(p + k * half, make_float2(o.x + v0, o.y + v1));
   }
 }
-// r = b - A x: on the black cells into r (blockIdx.z = plane), or, TAKE, on
-// all cells into b itself with sum += x (blockIdx.z = 2 plane + colour).
+// r = b - A x after sweeps that end on the red cells, whose residual is zero:
+//   kResidual  the black cells into r (blockIdx.z = plane)
+//   kTake      the black cells into r, zeros on the red ones, and sum += x
+//              (blockIdx.z = 2 plane + colour)
+//   kTakeOne   as kTake after one sweep from zero that divides: a black cell's
+//              residual is what its red neighbours then changed
+//   kTaken     as kTake where r's black cells hold the residual already
 // Four cells of a row per thread as in k_rbgs_v4 (rows with nx % 8 == 0), or
 // one (VEC = 1).
-template <bool TAKE, int VEC>
+enum ResidualMode { kResidual, kTake, kTakeOne, kTaken };
+template <int VEC> struct RowCells { float v[VEC]; };
+template <int VEC>
+__device__ __forceinline__ RowCells<VEC> ld_cells(const float* a, bool on) {
+  RowCells<VEC> o;
+  if (VEC == 4) {
+    const float4 f = on ? *reinterpret_cast<const float4*>(a) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    o.v[0] = f.x; o.v[VEC > 1 ? 1 : 0] = f.y; o.v[VEC > 2 ? 2 : 0] = f.z; o.v[VEC > 3 ? 3 : 0] = f.w;
+  } else {
+    o.v[0] = on ? *a : 0.0f;
+  }
+  return o;
+}
+template <int VEC>
+__device__ __forceinline__ void st_cells(float* a, const RowCells<VEC>& v) {
+  if (VEC == 4)
+    *reinterpret_cast<float4*>(a) = make_float4(v.v[0], v.v[VEC > 1 ? 1 : 0], v.v[VEC > 2 ? 2 : 0], v.v[VEC > 3 ? 3 : 0]);
+  else
+    *a = v.v[0];
+}
+template <int MODE, int VEC>
 __global__ void __launch_bounds__(256) k_residual_t(Grid d, float inv_h2, int ref, const float* __restrict__ x,
                                                     const float* b, float* r, float* __restrict__ sum) {
   pdl_wait();
@@ -654,34 +679,35 @@ __global__ void __launch_bounds__(256) k_residual_t(Grid d, float inv_h2, int re
   const uint32_t hx = (uint32_t)d.nx >> 1, half = (uint32_t)(d.n() >> 1), sz = (uint32_t)d.ny * hx;
   const uint32_t k0 = (blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int z = TAKE ? blockIdx.z >> 1 : blockIdx.z, color = TAKE ? blockIdx.z & 1 : 1;
+  const int z = MODE == kResidual ? blockIdx.z : blockIdx.z >> 1, color = MODE == kResidual ? 1 : blockIdx.z & 1;
   if (k0 >= hx || y >= d.ny) return;
   const uint32_t own = color ? half : 0u, oth = color ? 0u : half;
   const uint32_t i = (uint32_t)z * sz + (uint32_t)y * hx + k0;
+  const RowCells<VEC> xc = ld_cells<VEC>(x + own + i, true);
+  if (MODE != kResidual) {
+    RowCells<VEC> sv = ld_cells<VEC>(sum + own + i, true);
+#pragma unroll
+    for (int j = 0; j < VEC; ++j) sv.v[j] = sv.v[j] + xc.v[j];
+    st_cells<VEC>(sum + own + i, sv);
+    if (color == 0) {
+      st_cells<VEC>(r + i, RowCells<VEC>{});
+      return;
+    }
+    if (MODE == kTaken) return;
+  }
   const bool has_ym = y > 0, has_yp = y < d.ny - 1, has_zm = z > 0, has_zp = z < d.nz - 1;
   const int p = (y + z + color) & 1;
   const bool has_e = p == 0 ? k0 > 0 : k0 + VEC < hx;  // the word before (p = 0) or after the others
   const float dyz = (has_ym ? 1.0f : 0.0f) + (has_yp || ref ? 1.0f : 0.0f) + (has_zm ? 1.0f : 0.0f) +
                     (has_zp ? 1.0f : 0.0f);
-  struct V { float v[VEC]; };
-  auto ld = [&](const float* a, bool on) {
-    V o;
-    if (VEC == 4) {
-      const float4 f = on ? *reinterpret_cast<const float4*>(a) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-      o.v[0] = f.x; o.v[VEC > 1 ? 1 : 0] = f.y; o.v[VEC > 2 ? 2 : 0] = f.z; o.v[VEC > 3 ? 3 : 0] = f.w;
-    } else {
-      o.v[0] = on ? *a : 0.0f;
-    }
-    return o;
-  };
   const float* xo = x + oth + i;
-  const V cm = ld(xo, true), ym = ld(has_ym ? xo - hx : xo, has_ym), yp = ld(has_yp ? xo + hx : xo, has_yp);
-  const V zm = ld(has_zm ? xo - sz : xo, has_zm), zp = ld(has_zp ? xo + sz : xo, has_zp);
+  const RowCells<VEC> cm = ld_cells<VEC>(xo, true), ym = ld_cells<VEC>(has_ym ? xo - hx : xo, has_ym),
+                      yp = ld_cells<VEC>(has_yp ? xo + hx : xo, has_yp),
+                      zm = ld_cells<VEC>(has_zm ? xo - sz : xo, has_zm),
+                      zp = ld_cells<VEC>(has_zp ? xo + sz : xo, has_zp);
   const float ex = has_e ? (p == 0 ? xo[-1] : xo[VEC]) : 0.0f;
-  const V xc = ld(x + own + i, true), bv = ld(b + own + i, true);
-  V sv = {};
-  if (TAKE) sv = ld(sum + own + i, true);
-  V out;
+  const RowCells<VEC> bv = ld_cells<VEC>(b + own + i, MODE != kTakeOne);
+  RowCells<VEC> out;
 #pragma unroll
   for (int j = 0; j < VEC; ++j) {
     const float xm = p == 0 ? (j == 0 ? ex : cm.v[j - (j > 0)]) : cm.v[j];
@@ -689,17 +715,56 @@ __global__ void __launch_bounds__(256) k_residual_t(Grid d, float inv_h2, int re
     const bool edge = !has_e && (p == 0 ? j == 0 : j == VEC - 1);
     const float diag = dyz + (edge ? 1.0f : 2.0f);
     const float sumN = ((((xm + xp) + ym.v[j]) + yp.v[j]) + zm.v[j]) + zp.v[j];
-    out.v[j] = bv.v[j] - (sumN - diag * xc.v[j]) * inv_h2;
-    if (TAKE) sv.v[j] = sv.v[j] + xc.v[j];
+    out.v[j] = MODE == kTakeOne ? -sumN * inv_h2 : bv.v[j] - (sumN - diag * xc.v[j]) * inv_h2;
   }
-  auto put = [&](float* a, const V& v) {
-    if (VEC == 4)
-      *reinterpret_cast<float4*>(a) = make_float4(v.v[0], v.v[VEC > 1 ? 1 : 0], v.v[VEC > 2 ? 2 : 0], v.v[VEC > 3 ? 3 : 0]);
-    else
-      *a = v.v[0];
+  st_cells<VEC>(r + own + i, out);
+}
+// The finest grid's step of the transposed cycle from the coarse correction ec
+// to the sweeps after it, in correction form: sum += x + ec / 8, and the
+// residual after that, r = r0 - A (ec / 8), the right-hand side of sweeps from
+// zero.  ec / 8 is constant on 2x2x2 cells (h^2 = 1 here), so a cell differs
+// from one neighbour per axis, and the residual never is the difference of two
+// large numbers: formed as ap - A x after sweeps of x itself it carried the
+// rounding of x (72x104x56, gradient of the first pressure against 64 bits:
+// 1.1e-5 of it, 1.2e-6 now, 3e-6 with the half-sweeps transposed one by one;
+// one launch more a cycle, 720 -> 727 us a backward step at 96x128x96).  BLACK: r0 is zero on the red cells.  blockIdx.z = 2
+// plane + colour; VEC as in k_residual_t.
+template <bool BLACK, int VEC>
+__global__ void __launch_bounds__(256) k_correct_t(Grid f, Grid c, int ref, const float* r0, float* r,
+                                                   const float* __restrict__ ec, const float* __restrict__ x,
+                                                   float* __restrict__ sum) {
+  pdl_wait();
+  pdl_trigger();
+  const int hx = f.nx >> 1;  // words of a fine row, cells of a coarse one
+  const int k0 = (int)(blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+  const int y = blockIdx.y * blockDim.y + threadIdx.y;
+  const int z = blockIdx.z >> 1, color = blockIdx.z & 1;
+  if (k0 >= hx || y >= f.ny) return;
+  const uint32_t half = (uint32_t)(f.n() >> 1), hc = (uint32_t)hx >> 1, halfc = (uint32_t)(c.n() >> 1);
+  const uint32_t i = (color ? half : 0u) + ((uint32_t)z * f.ny + (uint32_t)y) * (uint32_t)hx + (uint32_t)k0;
+  const int p = (y + z + color) & 1;  // the cells are x = 2k + p: their parents are the coarse row's cells k
+  const int Y = y >> 1, Z = z >> 1;
+  auto at = [&](int X, int Yc, int Zc) {
+    return ec[(((X + Yc + Zc) & 1) ? halfc : 0u) + ((uint32_t)Zc * c.ny + (uint32_t)Yc) * hc + (uint32_t)(X >> 1)];
   };
-  put(r + own + i, out);
-  if (TAKE) put(sum + own + i, sv);
+  // each axis' neighbour with another parent, or the parent itself at a wall
+  const int Yn = y & 1 ? min(Y + 1, c.ny - 1) : max(Y - 1, 0), Zn = z & 1 ? min(Z + 1, c.nz - 1) : max(Z - 1, 0);
+  const bool top = ref && y == f.ny - 1;  // Dirichlet: a zero above
+  float e[VEC + 1];  // parents k0 - 1 + p .. k0 + VEC - 1 + p
+#pragma unroll
+  for (int j = 0; j <= VEC; ++j) e[j] = at(dob_clampi(k0 - 1 + p + j, 0, hx - 1), Y, Z);
+  const bool have = !BLACK || color == 1;
+  const RowCells<VEC> rv = ld_cells<VEC>(r0 + (have ? i : 0u), have), xv = ld_cells<VEC>(x + i, true);
+  RowCells<VEC> sv = ld_cells<VEC>(sum + i, true), out;
+#pragma unroll
+  for (int j = 0; j < VEC; ++j) {
+    const float own = p == 0 ? e[j + 1] : e[j], en = p == 0 ? e[j] : e[j + 1];
+    const float ey = top ? 0.0f : at(k0 + j, Yn, Z), ez = at(k0 + j, Y, Zn);
+    out.v[j] = rv.v[j] - 0.125f * (((en - own) + (ey - own)) + (ez - own));
+    sv.v[j] = sv.v[j] + (xv.v[j] + 0.125f * own);
+  }
+  st_cells<VEC>(r + i, out);
+  st_cells<VEC>(sum + i, sv);
 }
 
 // Exact coarsest-grid solve e = M b with the dense symmetric inverse M
@@ -1517,7 +1582,7 @@ static void half_sweep_v4(const DevState& s, const MgLevel& L, int c, bool divid
   const dim3 bq = quad_block(L.d);
   dim3 gq = quad_grid(L.d, bq);
   const size_t threads = (L.d.n() >> 1) / 4, wave2 = (size_t)s.num_sms * 2048;
-  if (divide) {  // the coarsest grid, at most 204800 cells
+  if (divide) {  // a coarsest grid of at most 204800 cells, or the only one
     launch_pdl(k_rbgs_v4<T, 1, ZOTH, true>, gq, bq, 0, st, L.d, c, L.h2, s.ref, own, oth, bown, skip);
   } else if (L.d.nz % 4 == 0 && threads / 4 >= wave2) {
     gq.z = L.d.nz / 4;
@@ -1672,76 +1737,91 @@ static void vcycle(const DevState& s, T* x0, const T* b0, T* const* E, T* const*
 // prolongation for a restriction, the transposed coarsest solve, the
 // transposed average for a prolongation, and the pre-smoothing's sweeps with
 // the colours exchanged.  So it runs on the forward cycle's kernels and level
-// arrays, one launch per leg on the small levels, and one residual pass ends
-// it (96x128x96, a backward step of four cycles: 969 -> 759 us against
-// half-sweeps transposed one by one, which update the right-hand side's
-// adjoint in every launch).  x0, t0: two arrays of the finest grid's size, R[l] one of every other
+// arrays, one launch per leg on the small levels (96x128x96, a backward step of
+// four cycles: 969 -> 727 us against half-sweeps transposed one by one,
+// which update the right-hand side's adjoint in every launch).  The finest
+// grid's last sweeps run on the residual, from zero (k_correct_t).
+// x0, t0: two arrays of the finest grid's size, R[l] one of every other
 // level's (residuals).
+static void residual_t(const DevState& s, int l, ResidualMode mode, const float* x, const float* b, float* r,
+                       float* sum, cudaStream_t st) {
+  const Grid& d = s.lv[l].d;
+  const bool vec = d.nx % 8 == 0;
+  const dim3 block = vec ? quad_block(d) : b_cells();
+  dim3 grid = vec ? quad_grid(d, block) : g_half(d);
+  if (mode != kResidual) grid.z = 2 * d.nz;
+  auto run = [&](auto* k) { launch_pdl(k, grid, block, 0, st, d, 1.0f / s.lv[l].h2, s.ref, x, b, r, sum); };
+  if (mode == kResidual) vec ? run(k_residual_t<kResidual, 4>) : run(k_residual_t<kResidual, 1>);
+  else if (mode == kTake) vec ? run(k_residual_t<kTake, 4>) : run(k_residual_t<kTake, 1>);
+  else if (mode == kTakeOne) vec ? run(k_residual_t<kTakeOne, 4>) : run(k_residual_t<kTakeOne, 1>);
+  else vec ? run(k_residual_t<kTaken, 4>) : run(k_residual_t<kTaken, 1>);
+}
 static void transposed_cycle(const DevState& s, float* ap, float* arhs, float* x0, float* t0, float* const* R,
                              cudaStream_t st) {
   const int L = s.nlev;
+  if (L == 1) {
+    // Each sweep on the residual of the one before, dividing: no other level damps
+    // the rounding of x, nor what the product with fl(1/6) leaves of a residual.
+    for (int k = 0; k < s.pre + s.post; ++k) {
+      smooth<float, float>(s, 0, x0, ap, 1, true, nullptr, nullptr, st, false, 1, true);
+      residual_t(s, 0, kTakeOne, x0, ap, ap, arhs, st);
+    }
+    return;
+  }
   float* X[kMaxLevels];
   const float* B[kMaxLevels];
   for (int l = 0; l < L; ++l) {
     X[l] = l ? s.lv[l].e : x0;
     B[l] = l ? s.lv[l].b : ap;
   }
-  if (L == 1) {
-    smooth<float, float>(s, 0, x0, ap, s.pre + s.post, true, nullptr, nullptr, st, false, 1);
-  } else {
-    for (int l = 0; l < L - 1; ++l) {
-      const Grid f = s.lv[l].d, c = s.lv[l + 1].d;
-      const int sweeps = l ? s.post : s.post0;
-      float* r = l ? R[l] : t0;
-      const float* from = r;
-      if (leg_ok(s, l)) {
-        leg_down<float, float>(s, l, nullptr, B[l], X[l], nullptr, sweeps, nullptr, st, r);
-      } else {
-        smooth<float, float>(s, l, X[l], B[l], sweeps, true, nullptr, nullptr, st, false, 1);
-        const float inv_h2 = 1.0f / s.lv[l].h2;
-        if (sweeps == 0) {
-          from = B[l];  // x = 0: the residual is the right-hand side
-        } else if (f.nx % 8 == 0) {
-          const dim3 bq = quad_block(f);
-          launch_pdl(k_residual_t<false, 4>, quad_grid(f, bq), bq, 0, st, f, inv_h2, s.ref, (const float*)X[l], B[l],
-                     r, (float*)nullptr);
-        } else {
-          launch_pdl(k_residual_t<false, 1>, g_half(f), b_cells(), 0, st, f, inv_h2, s.ref, (const float*)X[l], B[l],
-                     r, (float*)nullptr);
-        }
-      }
-      const dim3 bp = pair_block(c);
-      if (sweeps > 0) launch_pdl(k_prolong_t2<true>, pair_grid(c, bp), bp, 0, st, f, c, s.ref, from, s.lv[l + 1].b);
-      else launch_pdl(k_prolong_t2<false>, pair_grid(c, bp), bp, 0, st, f, c, s.ref, from, s.lv[l + 1].b);
+  for (int l = 0; l < L - 1; ++l) {
+    const Grid f = s.lv[l].d, c = s.lv[l + 1].d;
+    const int sweeps = l ? s.post : s.post0;
+    float* r = l ? R[l] : t0;
+    if (leg_ok(s, l)) {
+      leg_down<float, float>(s, l, nullptr, B[l], X[l], nullptr, sweeps, nullptr, st, r);
+    } else {
+      smooth<float, float>(s, l, X[l], B[l], sweeps, true, nullptr, nullptr, st, false, 1);
+      if (sweeps > 0) residual_t(s, l, kResidual, X[l], B[l], r, nullptr, st);
     }
-    coarse_solve<float>(s, L - 1, X[L - 1], B[L - 1], nullptr, st, 1);
-    for (int l = L - 2; l >= 0; --l) {
-      const Grid f = s.lv[l].d, c = s.lv[l + 1].d;
-      const int sweeps = l ? s.pre : s.pre0;
-      if (leg_ok(s, l)) {
-        float* out = l ? s.lv[l].e2 : t0;
-        leg_up<float, float>(s, l, X[l], B[l], X[l + 1], out, sweeps, nullptr, st, true);
-        X[l] = out;
-        continue;
-      }
-      const dim3 bp = pair_block(c);
-      const dim3 gp((c.nx / 2 + bp.x - 1) / bp.x, (f.ny + bp.y - 1) / bp.y, f.nz);
-      if (sweeps > 0) launch_pdl(k_inject_t2<true>, gp, bp, 0, st, f, c, X[l], (const float*)X[l + 1]);
-      else launch_pdl(k_inject_t2<false>, gp, bp, 0, st, f, c, X[l], (const float*)X[l + 1]);
-      smooth<float, float>(s, l, X[l], B[l], sweeps, false, nullptr, nullptr, st, false, 1);
-    }
+    const dim3 bp = pair_block(c);
+    // without sweeps x = 0: the residual is the right-hand side
+    if (sweeps > 0) launch_pdl(k_prolong_t2<true>, pair_grid(c, bp), bp, 0, st, f, c, s.ref, (const float*)r, s.lv[l + 1].b);
+    else launch_pdl(k_prolong_t2<false>, pair_grid(c, bp), bp, 0, st, f, c, s.ref, B[l], s.lv[l + 1].b);
   }
-  const Grid d = s.g;
-  if (d.nx % 8 == 0) {
-    const dim3 bq = quad_block(d);
-    dim3 gq = quad_grid(d, bq);
-    gq.z = 2 * d.nz;
-    launch_pdl(k_residual_t<true, 4>, gq, bq, 0, st, d, 1.0f, s.ref, (const float*)X[0], (const float*)ap, ap, arhs);
+  coarse_solve<float>(s, L - 1, X[L - 1], B[L - 1], nullptr, st, 1);
+  for (int l = L - 2; l >= 1; --l) {
+    const Grid f = s.lv[l].d, c = s.lv[l + 1].d;
+    if (leg_ok(s, l)) {
+      leg_up<float, float>(s, l, X[l], B[l], X[l + 1], s.lv[l].e2, s.pre, nullptr, st, true);
+      X[l] = s.lv[l].e2;
+      continue;
+    }
+    const dim3 bp = pair_block(c);
+    const dim3 gp((c.nx / 2 + bp.x - 1) / bp.x, (f.ny + bp.y - 1) / bp.y, f.nz);
+    if (s.pre > 0) launch_pdl(k_inject_t2<true>, gp, bp, 0, st, f, c, X[l], (const float*)X[l + 1]);
+    else launch_pdl(k_inject_t2<false>, gp, bp, 0, st, f, c, X[l], (const float*)X[l + 1]);
+    smooth<float, float>(s, l, X[l], B[l], s.pre, false, nullptr, nullptr, st, false, 1);
+  }
+  const Grid d = s.g, c = s.lv[1].d;
+  const bool vec = d.nx % 8 == 0, black = s.post0 > 0;
+  const dim3 block = vec ? quad_block(d) : b_cells();
+  dim3 grid = vec ? quad_grid(d, block) : g_half(d);
+  grid.z = 2 * d.nz;
+  float* r1 = s.pre0 > 0 ? t0 : ap;  // in place of what it reads, or the result
+  auto correct = [&](auto* k) {
+    launch_pdl(k, grid, block, 0, st, d, c, s.ref, black ? (const float*)t0 : (const float*)ap, r1, (const float*)X[1],
+               (const float*)x0, arhs);
+  };
+  if (black) vec ? correct(k_correct_t<true, 4>) : correct(k_correct_t<true, 1>);
+  else vec ? correct(k_correct_t<false, 4>) : correct(k_correct_t<false, 1>);
+  if (s.pre0 == 0) return;
+  if (leg_ok(s, 0)) {
+    leg_down<float, float>(s, 0, nullptr, t0, x0, nullptr, s.pre0, nullptr, st, ap);
+    residual_t(s, 0, kTaken, x0, t0, ap, arhs, st);
   } else {
-    dim3 gh = g_half(d);
-    gh.z = 2 * d.nz;
-    launch_pdl(k_residual_t<true, 1>, gh, b_cells(), 0, st, d, 1.0f, s.ref, (const float*)X[0], (const float*)ap, ap,
-               arhs);
+    smooth<float, float>(s, 0, x0, t0, s.pre0, true, nullptr, nullptr, st, false, 1);
+    residual_t(s, 0, kTake, x0, t0, ap, arhs, st);
   }
 }
 void launch_transposed_cycles(const DevState& s, float* ap, float* arhs, float* x0, float* t0, float* const* R,
